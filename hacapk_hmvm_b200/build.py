@@ -61,7 +61,7 @@ def hmvm_sources() -> list[str]:
 
 
 def hmvm_deps() -> list[str]:
-    deps = hmvm_sources() + [os.path.join(CSRC, f) for f in ("kernels.cuh", "kernels_multi.cuh", "kernels_tc.cuh", "kernels_tcw.cuh", "layout.hpp", "numfmt.hpp", "validate.hpp")]
+    deps = hmvm_sources() + [os.path.join(CSRC, f) for f in ("kernels.cuh", "kernels_multi.cuh", "kernels_dmma.cuh", "kernels_batch.cuh", "kernels_tc.cuh", "kernels_tcw.cuh", "layout.hpp", "numfmt.hpp", "validate.hpp")]
     deps += [os.path.join(INCLUDE, "hmvm_b200.h"), os.path.join(INCLUDE, "hacapk_hgen.h")]
     return deps
 

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "hmvm_b200.h"
+#include "kernels_batch.cuh"
 #include "kernels_tc.cuh"
 #include "kernels_tcw.cuh"
 #include "layout.hpp"
@@ -207,6 +208,10 @@ struct hmvm_plan {
   int64_t stage1_bytes = 0, stage2_bytes = 0;
   // multi-RHS (nrhs_max > 1): packed inputs, t and partial sums for up to nrhs_max rhs
   int nrhs_max = 1;
+  int32_t* d_segfirst = nullptr;  // per segment: first padded column within its item
+  int32_t* d_tbm1 = nullptr;      // team ranges of hmvm_dmma_kernel (its own warps per SM)
+  int32_t* d_tbm2 = nullptr;
+  int32_t mteams1 = 0, mteams2 = 0;
   double* d_xm64 = nullptr;
   float* d_xm32 = nullptr;
   void* d_tm = nullptr;
@@ -272,7 +277,8 @@ void free_plan_buffers(hmvm_plan* p) {
                   p->d_scale, p->d_xm64, p->d_xm32, p->d_tm,  p->d_pm,   p->d_xh,      p->d_yh,
                   p->d_xplanes, p->d_tplanes, p->d_scal, p->d_amax, p->d_xpl, p->d_tpl,
                   p->d_tscale, p->d_xscale, p->d_amax128, p->d_part, p->d_tblocks, p->d_tgroups,
-                  p->d_tops, p->d_tgfirst};
+                  p->d_tops, p->d_tgfirst, p->d_segfirst,
+                  p->d_tbm1, p->d_tbm2};
   for (void* b : bufs)
     if (b) cudaFree(b);
 }
@@ -310,6 +316,7 @@ int upload(Buf** dst, const void* src, size_t bytes, int64_t* total) {
 }
 
 int plan_mode(const hmvm_plan* p);
+int multi_smem(int mode);
 template <bool VST>
 MultiFn multi_kernel_for(int mode, int nr, int cfg);
 int tc_prepare(const hmvm_plan* p);
@@ -324,7 +331,7 @@ int prepare_kernels(const hmvm_plan* p) {
     int rc = tc_prepare(p);
     if (rc) return rc;
   } else if (p->nrhs_max > 1) {
-    const int smem = multi_smem_bytes(kMultiCfgs[kDefaultMultiCfg], plan_mode(p) == kModePlain64);
+    const int smem = multi_smem(plan_mode(p));
     for (int nr : {2, 4, 8})
       for (MultiFn f : {multi_kernel_for<true>(plan_mode(p), nr, kDefaultMultiCfg),
                         multi_kernel_for<false>(plan_mode(p), nr, kDefaultMultiCfg)})
@@ -504,6 +511,37 @@ int validate_layout(const HostLayout& L, std::string& msg) {
   return HMVM_OK;
 }
 
+// Items [first, end), in their stored order, cut into n ranges whose largest
+// cost (bytes and kDmmaItemOverhead per item) is as small as whole items allow.
+std::vector<int32_t> even_ranges(const HostLayout& L, int32_t first, int32_t end, int n) {
+  auto cost = [&](int32_t i) { return (int64_t)L.tiles[i].nvec * L.tiles[i].nrows * 16 + kDmmaItemOverhead; };
+  int64_t lo = 0, hi = 0;
+  for (int32_t i = first; i < end; i++) {
+    lo = std::max(lo, cost(i));
+    hi += cost(i);
+  }
+  lo = std::max(lo, hi / n);
+  auto cut = [&](int64_t cap, std::vector<int32_t>* out) {  // ranges of at most cap
+    int used = 0;
+    int32_t i = first;
+    while (i < end) {
+      if (out) out->push_back(i);
+      used++;
+      for (int64_t c = cost(i++); i < end && c + cost(i) <= cap; i++) c += cost(i);
+    }
+    return used;
+  };
+  while (lo < hi) {
+    const int64_t mid = lo + (hi - lo) / 2;
+    if (cut(mid, nullptr) <= n) hi = mid;
+    else lo = mid + 1;
+  }
+  std::vector<int32_t> out;
+  cut(hi, &out);
+  out.resize((size_t)n + 1, end);
+  return out;
+}
+
 int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** out, int sms_cap = 0) {
   if (!out) return set_error(HMVM_EINVAL, "plan output pointer is NULL");
   *out = nullptr;
@@ -640,6 +678,22 @@ int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** 
       if (!rc) rc = upload(&p->d_scale, L->rowscale.data(), L->rowscale.size() * sizeof(double), nullptr);
     }
     if (!rc && p->tcw) rc = tcw_buffers(p, *L);
+    if (!rc && p->nrhs_max > 1 && !p->tcw && !p->mixed) {
+      std::vector<int32_t> first(L->segs.size());
+      for (const hmvm_tile_desc& d : L->tiles) {
+        int32_t c = 0;
+        for (int32_t s = d.seg_begin; s < d.seg_begin + d.nseg; s++) {
+          first[s] = c;
+          c += (L->segs[s].ncols + L->vec - 1) / L->vec * L->vec;
+        }
+      }
+      rc = upload(&p->d_segfirst, first.data(), first.size() * 4, nullptr);
+      p->mteams1 = p->mteams2 = lsms * kDmmaWarpsPerSm;
+      const std::vector<int32_t> t1 = even_ranges(*L, 0, L->stage1_tiles, p->mteams1);
+      const std::vector<int32_t> t2 = even_ranges(*L, L->stage1_tiles, (int32_t)L->tiles.size(), p->mteams2);
+      if (!rc) rc = upload(&p->d_tbm1, t1.data(), t1.size() * 4, nullptr);
+      if (!rc) rc = upload(&p->d_tbm2, t2.data(), t2.size() * 4, nullptr);
+    }
     if (!rc && p->nrhs_max > 1 && !p->tcw) {
       const size_t nr = (size_t)p->nrhs_max;
       cudaError_t e = cudaSuccess;
@@ -837,7 +891,9 @@ MultiFn multi_kernel_cfg(int cfg) {
   static_assert(kNumMultiCfgs == 1 && kDefaultMultiCfg == 0, "one multi-RHS shape is instantiated");
   (void)cfg;
   constexpr MultiCfg c = kMultiCfgs[kDefaultMultiCfg];
-  return hmvm_multi_kernel<c.wpb, c.slots, c.chunk, NR, MODE, VST>;
+  if constexpr (MODE == kModePlain64)
+    return hmvm_dmma_kernel<double, kDmmaCfg.wpb, kDmmaCfg.slots, kDmmaCfg.chunk, NR, VST>;
+  else return hmvm_multi_kernel<c.wpb, c.slots, c.chunk, NR, MODE, VST>;
 }
 template <int MODE, bool VST>
 MultiFn multi_kernel_nr(int nr, int cfg) {
@@ -889,6 +945,19 @@ void launch_pack(const hmvm_plan* p, const void* X, int64_t ldx, int nr, cudaStr
                                                            x32);
 }
 
+// Launch shape of the multi-RHS kernel of a mode: warps per CTA and shared memory.
+int multi_wpb(int mode) { return mode == kModePlain64 ? kDmmaCfg.wpb : kMultiCfgs[kDefaultMultiCfg].wpb; }
+int multi_smem(int mode) {
+  return mode == kModePlain64 ? dmma_smem_bytes(kDmmaCfg) : multi_smem_bytes(kMultiCfgs[kDefaultMultiCfg], false);
+}
+
+// The team ranges of a stage's multi-RHS kernel.
+void multi_teams(const hmvm_plan* p, bool vst, MultiArgs& a) {
+  const bool own = p->d_tbm1 != nullptr;
+  a.team_begin = own ? (vst ? p->d_tbm1 : p->d_tbm2) : (vst ? p->d_tb1 : p->d_tb2);
+  a.nteams = own ? (vst ? p->mteams1 : p->mteams2) : (vst ? p->stage1_teams : p->stage2_teams);
+}
+
 // One pass: nr (<= nr_inst) right-hand sides X[:, 0:nr] -> Y[:, 0:nr].
 int launch_multi_stages(hmvm_plan* p, void* Y, int64_t ldy, int nr, int nr_inst, cudaStream_t st);
 
@@ -919,9 +988,9 @@ int launch_multi_stages(hmvm_plan* p, void* Y, int64_t ldy, int nr, int nr_inst,
   a.p = p->d_pm;
   a.out_idx = p->d_out_idx;
   a.scale = p->d_scale;
+  a.seg_first = p->d_segfirst;
   const int mode = plan_mode(p);
-  const MultiCfg& c = kMultiCfgs[kDefaultMultiCfg];
-  const int threads = 32 * c.wpb, smem = multi_smem_bytes(c, mode == kModePlain64);
+  const int wpb = multi_wpb(mode), threads = 32 * wpb, smem = multi_smem(mode);
   cudaEvent_t* ev = nullptr;
   if (p->profiling && p->prof_count < kMaxProfiled) {
     ev = &p->prof_events[kEventsPerApply * (size_t)p->prof_count];
@@ -929,9 +998,8 @@ int launch_multi_stages(hmvm_plan* p, void* Y, int64_t ldy, int nr, int nr_inst,
   }
   if (ev) cudaEventRecord(ev[0], st);
   if (p->stage1_tiles > 0) {
-    a.team_begin = p->d_tb1;
-    a.nteams = p->stage1_teams;
-    const int ctas = (p->stage1_teams + c.wpb - 1) / c.wpb;
+    multi_teams(p, true, a);
+    const int ctas = (a.nteams + wpb - 1) / wpb;
     multi_kernel_for<true>(mode, nr_inst, kDefaultMultiCfg)<<<ctas, threads, smem, st>>>(a);
     HMVM_CUDA_TRY(cudaGetLastError(), "multi-RHS V-stage launch");
   }
@@ -945,9 +1013,8 @@ int launch_multi_stages(hmvm_plan* p, void* Y, int64_t ldy, int nr, int nr_inst,
   }
   if (ev) cudaEventRecord(ev[2], st);
   {
-    a.team_begin = p->d_tb2;
-    a.nteams = p->stage2_teams;
-    const int ctas = (p->stage2_teams + c.wpb - 1) / c.wpb;
+    multi_teams(p, false, a);
+    const int ctas = (a.nteams + wpb - 1) / wpb;
     multi_kernel_for<false>(mode, nr_inst, kDefaultMultiCfg)<<<ctas, threads, smem, st>>>(a);
     HMVM_CUDA_TRY(cudaGetLastError(), "multi-RHS row-stage launch");
   }
@@ -1146,11 +1213,17 @@ int tcw_kernels_per_pass(const hmvm_plan* p) {
   return (p->tcw_bf ? 1 : 2) + (p->stage1_tiles > 0) + (p->n_red1 > 0) + 1;
 }
 
-// Right-hand sides per pass: the largest of 8, 4, 2 that is <= nrhs_max and
-// not above what is left (a last single column runs in a 2-wide pass).
-int multi_pass_width(int nrhs_max, int left) {
+// Right-hand sides per pass, of 8, 4 and 2.  FP64 plans: the narrowest width up
+// to nrhs_max that takes all that is left, else the widest, since a pass costs
+// about the same at every width (the matrix stream).  Others: the widest up to
+// nrhs_max that is not above what is left (a last single column runs in a
+// 2-wide pass).
+int multi_pass_width(const hmvm_plan* p, int left) {
+  if (plan_mode(p) == kModePlain64)
+    for (int w : {2, 4, 8})
+      if (w <= p->nrhs_max && w >= left) return w;
   for (int w : {8, 4, 2})
-    if (w <= nrhs_max && w <= std::max(left, 2)) return w;
+    if (w <= p->nrhs_max && w <= std::max(left, 2)) return w;
   return 2;
 }
 
@@ -1161,7 +1234,7 @@ struct Pass {
 std::vector<Pass> multi_passes(const hmvm_plan* p, int nrhs) {
   std::vector<Pass> v;
   for (int r0 = 0; r0 < nrhs;) {
-    const int w = p->tcw ? kTcwRhs : p->nrhs_max <= 1 ? 1 : p->tc ? kTcNrhs : multi_pass_width(p->nrhs_max, nrhs - r0);
+    const int w = p->tcw ? kTcwRhs : p->nrhs_max <= 1 ? 1 : p->tc ? kTcNrhs : multi_pass_width(p, nrhs - r0);
     const int nr = std::min(w, nrhs - r0);
     v.push_back(Pass{r0, nr, w});
     r0 += nr;
@@ -1565,7 +1638,7 @@ int hmvm_b200_plan_multi_kernel_count(const hmvm_plan* p, int32_t nrhs) {
   if (p->tc)  // per pass: pack, 2 x (max, planes), the stages and their reductions
     return (nrhs + kTcNrhs - 1) / kTcNrhs * (5 + (p->stage1_tiles > 0) + (p->n_red1 > 0) + 1 + (p->n_red2 > 0));
   int passes = 0;
-  for (int r0 = 0; r0 < nrhs; passes++) r0 += std::min(multi_pass_width(p->nrhs_max, nrhs - r0), nrhs - r0);
+  for (int r0 = 0; r0 < nrhs; passes++) r0 += std::min(multi_pass_width(p, nrhs - r0), nrhs - r0);
   return passes * (1 + (p->stage1_tiles > 0) + (p->n_red1 > 0) + 1 + (p->n_red2 > 0));
 }
 
@@ -2040,7 +2113,7 @@ int batch_mode(const hmvm_batch* b) { return plan_mode(b->cls.front().plan); }
 
 template <int MODE, bool VST>
 const void* batch_stage_kernel() {
-  constexpr MultiCfg c = kMultiCfgs[kDefaultMultiCfg];
+  constexpr MultiCfg c = MODE == kModePlain64 ? kDmmaCfg : kMultiCfgs[kDefaultMultiCfg];
   return (const void*)hmvm_batch_multi_kernel<c.wpb, c.slots, c.chunk, MODE, VST>;
 }
 const void* batch_stage_kernel_for(int mode, bool vst) {
@@ -2122,7 +2195,7 @@ int batch_create(const std::vector<LeafTable>& tabs, bool is_float, const hmvm_p
   b->device = b->cls.front().plan->device;
   {
     DeviceGuard g(b->device);
-    const int smem = multi_smem_bytes(kMultiCfgs[kDefaultMultiCfg], batch_mode(b) == kModePlain64);
+    const int smem = multi_smem(batch_mode(b));
     for (bool vst : {true, false}) {
       cudaError_t e = cudaFuncSetAttribute(batch_stage_kernel_for(batch_mode(b), vst),
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -2147,8 +2220,7 @@ MultiArgs part_args(const hmvm_plan* p, const PassBufs& q, bool vst, int64_t ldy
   a.err = p->d_err;
   a.tiles = p->d_tiles;
   a.segs = p->d_segs;
-  a.team_begin = vst ? p->d_tb1 : p->d_tb2;
-  a.nteams = vst ? p->stage1_teams : p->stage2_teams;
+  multi_teams(p, vst, a);
   a.data = p->d_data;
   a.x64 = q.xm64;
   a.x32 = q.xm32;
@@ -2159,6 +2231,7 @@ MultiArgs part_args(const hmvm_plan* p, const PassBufs& q, bool vst, int64_t ldy
   a.p = q.pm;
   a.out_idx = p->d_out_idx;
   a.scale = p->d_scale;
+  a.seg_first = p->d_segfirst;
   return a;
 }
 
@@ -2191,13 +2264,12 @@ int batch_set_io(hmvm_batch* b, const void* const* X, const int64_t* ldx, void* 
   std::vector<BatchPart> p1, p2;
   std::vector<BatchRedPart> r1, r2;
   int64_t nmax_rows = 0;
-  auto stage_add = [](std::vector<BatchPart>& v, const MultiArgs& a, int nr) {
-    const int ctas = (a.nteams + kMultiCfgs[kDefaultMultiCfg].wpb - 1) / kMultiCfgs[kDefaultMultiCfg].wpb;
-    if (ctas <= 0) return;
+  const int wpb = multi_wpb(batch_mode(b));
+  auto stage_add = [wpb](std::vector<BatchPart>& v, const MultiArgs& a, int nr) {
+    if (a.nteams <= 0) return;
     BatchPart q;
     q.a = a;
-    q.cta0 = v.empty() ? 0 : v.back().cta0 + (v.back().a.nteams + kMultiCfgs[kDefaultMultiCfg].wpb - 1) /
-                                                  kMultiCfgs[kDefaultMultiCfg].wpb;
+    q.cta0 = v.empty() ? 0 : v.back().cta0 + (v.back().a.nteams + wpb - 1) / wpb;
     q.nr = nr;
     v.push_back(q);
   };
@@ -2290,8 +2362,7 @@ int batch_run_t(hmvm_batch* b, cudaStream_t st) {
   if (b->pack.empty()) return HMVM_OK;
   const int mode = batch_mode(b);
   int* err = b->cls.front().plan->d_err;
-  const MultiCfg& mc = kMultiCfgs[kDefaultMultiCfg];
-  const int threads = 32 * mc.wpb, smem = multi_smem_bytes(mc, mode == kModePlain64);
+  const int wpb = multi_wpb(mode), threads = 32 * wpb, smem = multi_smem(mode);
   const unsigned gx = (unsigned)std::max<int64_t>(1, std::min<int64_t>((b->nmax_rows * 8 + 255) / 256, 64));
   const dim3 pgrid(gx, (unsigned)b->pack.size());
   const int nio = (int)b->io.size();
@@ -2315,7 +2386,7 @@ int batch_run_t(hmvm_batch* b, cudaStream_t st) {
   auto run_stage = [&](int k0, int n, bool vst) -> int {
     if (n == 0) return HMVM_OK;
     const BatchPart& last = b->parts[k0 + n - 1];
-    const unsigned grid = (unsigned)(last.cta0 + (last.a.nteams + mc.wpb - 1) / mc.wpb);
+    const unsigned grid = (unsigned)(last.cta0 + (last.a.nteams + wpb - 1) / wpb);
     const BatchPart* dp = b->d_parts + k0;
     void* args[] = {(void*)&dp, (void*)&n};
     HMVM_CUDA_TRY(cudaLaunchKernel(batch_stage_kernel_for(mode, vst), dim3(grid), dim3((unsigned)threads), args,

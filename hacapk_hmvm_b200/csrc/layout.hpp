@@ -185,6 +185,22 @@ inline int multi_smem_bytes(const MultiCfg& c, bool f64) {
   return c.wpb * (c.slots * c.chunk + 2 * multi_zbytes(f64) + c.slots * 8);
 }
 constexpr int kDefaultMultiCfg = 0;
+// hmvm_dmma_kernel: 3 CTAs of 4 warps per SM; per warp a ring of 2 x 4 KiB, the
+// copy of its first bytes (one vector of 32 rows) and two pages of inputs.  At
+// N = 65,536 FP64 with 8 right-hand sides, both stages: 12 warps 209 us; 8 warps
+// with rings of 2 x 8 KiB 212; 16 warps with pages of 2 KiB 214; 12 warps with
+// rings of 4 x 2 KiB 242 (every bulk copy costs the TMA unit some 20 cycles);
+// without the L2 prefetch of the next chunk 241.
+constexpr MultiCfg kDmmaCfg = {4, 2, 4096};
+constexpr int kDmmaPageBytes = 4096;
+constexpr int kDmmaRingPad = 512;
+constexpr int kDmmaWarpsPerSm = 12;
+// An item's fixed cost in bytes when the kernel's warps are given their items
+// (1.1 us per item against 6 us for the 21 KB of an average one).
+constexpr int64_t kDmmaItemOverhead = 4096;
+constexpr int dmma_smem_bytes(const MultiCfg& c) {
+  return c.wpb * (c.slots * c.chunk + kDmmaRingPad + 2 * kDmmaPageBytes + (c.slots + 2) * 8);
+}
 constexpr int kMultiWarpsPerSm = 12;    // resident warps (teams) per SM of the multi-RHS kernel
 constexpr int kMultiWarpsPerSmF64 = 8;  // the same for FP64 plans (8 KiB input buffers)
 
