@@ -208,10 +208,15 @@ struct hmvm_plan {
   int64_t stage1_bytes = 0, stage2_bytes = 0;
   // multi-RHS (nrhs_max > 1): packed inputs, t and partial sums for up to nrhs_max rhs
   int nrhs_max = 1;
+  // plain plans: hmvm_dmma_kernel's items, segments, team ranges and reductions
+  hmvm_tile_desc* d_mtiles = nullptr;
+  hmvm_seg_desc* d_msegs = nullptr;
   int32_t* d_segfirst = nullptr;  // per segment: first padded column within its item
-  int32_t* d_tbm1 = nullptr;      // team ranges of hmvm_dmma_kernel (its own warps per SM)
+  int32_t* d_tbm1 = nullptr;
   int32_t* d_tbm2 = nullptr;
-  int32_t mteams1 = 0, mteams2 = 0;
+  int4* d_mred1 = nullptr;
+  int4* d_mred2 = nullptr;
+  int32_t mteams1 = 0, mteams2 = 0, n_mred1 = 0, n_mred2 = 0;
   double* d_xm64 = nullptr;
   float* d_xm32 = nullptr;
   void* d_tm = nullptr;
@@ -278,7 +283,7 @@ void free_plan_buffers(hmvm_plan* p) {
                   p->d_xplanes, p->d_tplanes, p->d_scal, p->d_amax, p->d_xpl, p->d_tpl,
                   p->d_tscale, p->d_xscale, p->d_amax128, p->d_part, p->d_tblocks, p->d_tgroups,
                   p->d_tops, p->d_tgfirst, p->d_segfirst,
-                  p->d_tbm1, p->d_tbm2};
+                  p->d_tbm1, p->d_tbm2, p->d_mtiles, p->d_msegs, p->d_mred1, p->d_mred2};
   for (void* b : bufs)
     if (b) cudaFree(b);
 }
@@ -317,6 +322,7 @@ int upload(Buf** dst, const void* src, size_t bytes, int64_t* total) {
 
 int plan_mode(const hmvm_plan* p);
 int multi_smem(int mode);
+int multi_inst_width(int precision, int w);
 template <bool VST>
 MultiFn multi_kernel_for(int mode, int nr, int cfg);
 int tc_prepare(const hmvm_plan* p);
@@ -511,37 +517,6 @@ int validate_layout(const HostLayout& L, std::string& msg) {
   return HMVM_OK;
 }
 
-// Items [first, end), in their stored order, cut into n ranges whose largest
-// cost (bytes and kDmmaItemOverhead per item) is as small as whole items allow.
-std::vector<int32_t> even_ranges(const HostLayout& L, int32_t first, int32_t end, int n) {
-  auto cost = [&](int32_t i) { return (int64_t)L.tiles[i].nvec * L.tiles[i].nrows * 16 + kDmmaItemOverhead; };
-  int64_t lo = 0, hi = 0;
-  for (int32_t i = first; i < end; i++) {
-    lo = std::max(lo, cost(i));
-    hi += cost(i);
-  }
-  lo = std::max(lo, hi / n);
-  auto cut = [&](int64_t cap, std::vector<int32_t>* out) {  // ranges of at most cap
-    int used = 0;
-    int32_t i = first;
-    while (i < end) {
-      if (out) out->push_back(i);
-      used++;
-      for (int64_t c = cost(i++); i < end && c + cost(i) <= cap; i++) c += cost(i);
-    }
-    return used;
-  };
-  while (lo < hi) {
-    const int64_t mid = lo + (hi - lo) / 2;
-    if (cut(mid, nullptr) <= n) hi = mid;
-    else lo = mid + 1;
-  }
-  std::vector<int32_t> out;
-  cut(hi, &out);
-  out.resize((size_t)n + 1, end);
-  return out;
-}
-
 int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** out, int sms_cap = 0) {
   if (!out) return set_error(HMVM_EINVAL, "plan output pointer is NULL");
   *out = nullptr;
@@ -647,6 +622,24 @@ int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** 
     p->stage1_bytes = (v_elems + (int64_t)lt.nd) * L->elem_size;
     p->stage2_bytes = (L->stored_elems - v_elems + 2 * (int64_t)lt.nd) * L->elem_size;
   }
+  // A plain multi-RHS plan's teams are hmvm_dmma_kernel's; the single-vector
+  // kernels take the same items in as many ranges as they have resident teams.
+  const bool plain_multi = !L->mtiles.empty();
+  std::vector<int32_t> tb1 = L->team_begin1, tb2 = L->team_begin2;
+  if (plain_multi) {
+    p->mteams1 = L->stage1_teams;
+    p->mteams2 = L->stage2_teams;
+    p->n_mred1 = (int32_t)(L->mred1.size() / 4);
+    p->n_mred2 = (int32_t)(L->mred2.size() / 4);
+    p->stage1_teams = lsms * p->ctas_per_sm * teams_per_cta(p->kernel, p->stage1_cfg);
+    p->stage2_teams = lsms * p->ctas2_per_sm * teams_per_cta(p->kernel, p->stage2_cfg);
+    std::vector<int64_t> cost;
+    for (const hmvm_tile_desc& d : L->tiles) cost.push_back((int64_t)d.nvec * d.nrows * 16 + kItemOverheadBytes);
+    const auto mid = cost.begin() + L->stage1_tiles;
+    tb1 = even_ranges(std::vector<int64_t>(cost.begin(), mid), p->stage1_teams);
+    tb2 = even_ranges(std::vector<int64_t>(mid, cost.end()), p->stage2_teams);
+    for (int32_t& b : tb2) b += L->stage1_tiles;
+  }
   {
     DeviceGuard g(dev);
     if (!g.ok) rc = set_error(HMVM_ECUDA, "cannot select the plan's device");
@@ -655,8 +648,8 @@ int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** 
     p->device_bytes = dbytes;
     if (!rc) rc = upload(&p->d_tiles, L->tiles.data(), L->tiles.size() * sizeof(hmvm_tile_desc), nullptr);
     if (!rc) rc = upload(&p->d_segs, L->segs.data(), L->segs.size() * sizeof(hmvm_seg_desc), nullptr);
-    if (!rc) rc = upload(&p->d_tb1, L->team_begin1.data(), L->team_begin1.size() * 4, nullptr);
-    if (!rc) rc = upload(&p->d_tb2, L->team_begin2.data(), L->team_begin2.size() * 4, nullptr);
+    if (!rc) rc = upload(&p->d_tb1, tb1.data(), tb1.size() * 4, nullptr);
+    if (!rc) rc = upload(&p->d_tb2, tb2.data(), tb2.size() * 4, nullptr);
     if (!rc) rc = upload(&p->d_out_idx, L->out_idx.data(), L->out_idx.size() * 4, nullptr);
     if (!rc) rc = upload(&p->d_red1, L->red1.data(), L->red1.size() * 4, nullptr);
     if (!rc) rc = upload(&p->d_red2, L->red2.data(), L->red2.size() * 4, nullptr);
@@ -678,24 +671,17 @@ int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** 
       if (!rc) rc = upload(&p->d_scale, L->rowscale.data(), L->rowscale.size() * sizeof(double), nullptr);
     }
     if (!rc && p->tcw) rc = tcw_buffers(p, *L);
-    if (!rc && p->nrhs_max > 1 && !p->tcw && !p->mixed) {
-      std::vector<int32_t> first(L->segs.size());
-      for (const hmvm_tile_desc& d : L->tiles) {
-        int32_t c = 0;
-        for (int32_t s = d.seg_begin; s < d.seg_begin + d.nseg; s++) {
-          first[s] = c;
-          c += (L->segs[s].ncols + L->vec - 1) / L->vec * L->vec;
-        }
-      }
-      rc = upload(&p->d_segfirst, first.data(), first.size() * 4, nullptr);
-      p->mteams1 = p->mteams2 = lsms * kDmmaWarpsPerSm;
-      const std::vector<int32_t> t1 = even_ranges(*L, 0, L->stage1_tiles, p->mteams1);
-      const std::vector<int32_t> t2 = even_ranges(*L, L->stage1_tiles, (int32_t)L->tiles.size(), p->mteams2);
-      if (!rc) rc = upload(&p->d_tbm1, t1.data(), t1.size() * 4, nullptr);
-      if (!rc) rc = upload(&p->d_tbm2, t2.data(), t2.size() * 4, nullptr);
+    if (!rc && plain_multi) {
+      if (!rc) rc = upload(&p->d_mtiles, L->mtiles.data(), L->mtiles.size() * sizeof(hmvm_tile_desc), nullptr);
+      if (!rc) rc = upload(&p->d_msegs, L->msegs.data(), L->msegs.size() * sizeof(hmvm_seg_desc), nullptr);
+      if (!rc) rc = upload(&p->d_segfirst, L->mseg_first.data(), L->mseg_first.size() * 4, nullptr);
+      if (!rc) rc = upload(&p->d_tbm1, L->mteam_begin1.data(), L->mteam_begin1.size() * 4, nullptr);
+      if (!rc) rc = upload(&p->d_tbm2, L->mteam_begin2.data(), L->mteam_begin2.size() * 4, nullptr);
+      if (!rc) rc = upload(&p->d_mred1, L->mred1.data(), L->mred1.size() * 4, nullptr);
+      if (!rc) rc = upload(&p->d_mred2, L->mred2.data(), L->mred2.size() * 4, nullptr);
     }
     if (!rc && p->nrhs_max > 1 && !p->tcw) {
-      const size_t nr = (size_t)p->nrhs_max;
+      const size_t nr = (size_t)multi_inst_width(p->precision, p->nrhs_max);
       cudaError_t e = cudaSuccess;
       if (p->precision != HMVM_FP32) e = cudaMalloc(&p->d_xm64, (size_t)(L->nd + 16) * nr * sizeof(double));
       if (e == cudaSuccess && p->precision != HMVM_FP64)
@@ -893,6 +879,8 @@ MultiFn multi_kernel_cfg(int cfg) {
   constexpr MultiCfg c = kMultiCfgs[kDefaultMultiCfg];
   if constexpr (MODE == kModePlain64)
     return hmvm_dmma_kernel<double, kDmmaCfg.wpb, kDmmaCfg.slots, kDmmaCfg.chunk, NR, VST>;
+  else if constexpr (MODE == kModePlain32)
+    return hmvm_dmma_kernel<float, kDmmaCfg.wpb, kDmmaCfg.slots, kDmmaCfg.chunk, NR < 4 ? 4 : NR, VST>;
   else return hmvm_multi_kernel<c.wpb, c.slots, c.chunk, NR, MODE, VST>;
 }
 template <int MODE, bool VST>
@@ -912,6 +900,9 @@ MultiFn multi_kernel_for(int mode, int nr, int cfg) {
     default: return multi_kernel_nr<kModeMixedBF16, VST>(nr, cfg);
   }
 }
+// Values per column that a pass of width w packs: FP32 plans at least 4, so that
+// a column's inputs are a multiple of 16 bytes (bulk copies).
+int multi_inst_width(int precision, int w) { return precision == HMVM_FP32 && w < 4 ? 4 : w; }
 int plan_mode(const hmvm_plan* p) {
   if (p->mixed) return p->mixed_kcode == 3 ? kModeMixedBF16 : kModeMixed16;
   return p->precision == HMVM_FP64 ? kModePlain64 : kModePlain32;
@@ -946,16 +937,27 @@ void launch_pack(const hmvm_plan* p, const void* X, int64_t ldx, int nr, cudaStr
 }
 
 // Launch shape of the multi-RHS kernel of a mode: warps per CTA and shared memory.
-int multi_wpb(int mode) { return mode == kModePlain64 ? kDmmaCfg.wpb : kMultiCfgs[kDefaultMultiCfg].wpb; }
+int multi_wpb(int mode) { return mode <= kModePlain32 ? kDmmaCfg.wpb : kMultiCfgs[kDefaultMultiCfg].wpb; }
 int multi_smem(int mode) {
-  return mode == kModePlain64 ? dmma_smem_bytes(kDmmaCfg) : multi_smem_bytes(kMultiCfgs[kDefaultMultiCfg], false);
+  return mode <= kModePlain32 ? dmma_smem_bytes(kDmmaCfg) : multi_smem_bytes(kMultiCfgs[kDefaultMultiCfg]);
 }
 
-// The team ranges of a stage's multi-RHS kernel.
-void multi_teams(const hmvm_plan* p, bool vst, MultiArgs& a) {
-  const bool own = p->d_tbm1 != nullptr;
+// The items, team ranges and reductions of a stage's multi-RHS kernel.
+void multi_items(const hmvm_plan* p, bool vst, MultiArgs& a) {
+  const bool own = p->d_mtiles != nullptr;
+  a.tiles = own ? p->d_mtiles : p->d_tiles;
+  a.segs = own ? p->d_msegs : p->d_segs;
+  a.seg_first = p->d_segfirst;
   a.team_begin = own ? (vst ? p->d_tbm1 : p->d_tbm2) : (vst ? p->d_tb1 : p->d_tb2);
   a.nteams = own ? (vst ? p->mteams1 : p->mteams2) : (vst ? p->stage1_teams : p->stage2_teams);
+}
+const int4* multi_red(const hmvm_plan* p, bool vst, int* n) {
+  if (p->d_mtiles) {
+    *n = vst ? p->n_mred1 : p->n_mred2;
+    return vst ? p->d_mred1 : p->d_mred2;
+  }
+  *n = vst ? p->n_red1 : p->n_red2;
+  return vst ? p->d_red1 : p->d_red2;
 }
 
 // One pass: nr (<= nr_inst) right-hand sides X[:, 0:nr] -> Y[:, 0:nr].
@@ -976,8 +978,6 @@ int launch_multi_pass(hmvm_plan* p, const void* X, int64_t ldx, void* Y, int64_t
 int launch_multi_stages(hmvm_plan* p, void* Y, int64_t ldy, int nr, int nr_inst, cudaStream_t st) {
   MultiArgs a;
   a.err = p->d_err;
-  a.tiles = p->d_tiles;
-  a.segs = p->d_segs;
   a.data = p->d_data;
   a.x64 = p->d_xm64;
   a.x32 = p->d_xm32;
@@ -988,7 +988,6 @@ int launch_multi_stages(hmvm_plan* p, void* Y, int64_t ldy, int nr, int nr_inst,
   a.p = p->d_pm;
   a.out_idx = p->d_out_idx;
   a.scale = p->d_scale;
-  a.seg_first = p->d_segfirst;
   const int mode = plan_mode(p);
   const int wpb = multi_wpb(mode), threads = 32 * wpb, smem = multi_smem(mode);
   cudaEvent_t* ev = nullptr;
@@ -998,30 +997,33 @@ int launch_multi_stages(hmvm_plan* p, void* Y, int64_t ldy, int nr, int nr_inst,
   }
   if (ev) cudaEventRecord(ev[0], st);
   if (p->stage1_tiles > 0) {
-    multi_teams(p, true, a);
+    multi_items(p, true, a);
     const int ctas = (a.nteams + wpb - 1) / wpb;
     multi_kernel_for<true>(mode, nr_inst, kDefaultMultiCfg)<<<ctas, threads, smem, st>>>(a);
     HMVM_CUDA_TRY(cudaGetLastError(), "multi-RHS V-stage launch");
   }
   if (ev) cudaEventRecord(ev[1], st);
   const bool f32 = p->precision == HMVM_FP32;
-  if (p->n_red1 > 0) {
-    if (mode == kModePlain64) launch_reduce_multi<double, double, true>(nr_inst, p->d_red1, p->n_red1, p->d_pm, p->d_tm, 0, nr, st);
-    else if (f32) launch_reduce_multi<float, float, true>(nr_inst, p->d_red1, p->n_red1, p->d_pm, p->d_tm, 0, nr, st);
-    else launch_reduce_multi<double, float, true>(nr_inst, p->d_red1, p->n_red1, p->d_pm, p->d_tm, 0, nr, st);
+  int n_red = 0;
+  const int4* red = multi_red(p, true, &n_red);
+  if (n_red > 0) {
+    if (mode == kModePlain64) launch_reduce_multi<double, double, true>(nr_inst, red, n_red, p->d_pm, p->d_tm, 0, nr, st);
+    else if (f32) launch_reduce_multi<float, float, true>(nr_inst, red, n_red, p->d_pm, p->d_tm, 0, nr, st);
+    else launch_reduce_multi<double, float, true>(nr_inst, red, n_red, p->d_pm, p->d_tm, 0, nr, st);
     HMVM_CUDA_TRY(cudaGetLastError(), "multi-RHS V-stage reduction launch");
   }
   if (ev) cudaEventRecord(ev[2], st);
   {
-    multi_teams(p, false, a);
+    multi_items(p, false, a);
     const int ctas = (a.nteams + wpb - 1) / wpb;
     multi_kernel_for<false>(mode, nr_inst, kDefaultMultiCfg)<<<ctas, threads, smem, st>>>(a);
     HMVM_CUDA_TRY(cudaGetLastError(), "multi-RHS row-stage launch");
   }
   if (ev) cudaEventRecord(ev[3], st);
-  if (p->n_red2 > 0) {
-    if (f32) launch_reduce_multi<float, float, false>(nr_inst, p->d_red2, p->n_red2, p->d_pm, Y, ldy, nr, st);
-    else launch_reduce_multi<double, double, false>(nr_inst, p->d_red2, p->n_red2, p->d_pm, Y, ldy, nr, st);
+  red = multi_red(p, false, &n_red);
+  if (n_red > 0) {
+    if (f32) launch_reduce_multi<float, float, false>(nr_inst, red, n_red, p->d_pm, Y, ldy, nr, st);
+    else launch_reduce_multi<double, double, false>(nr_inst, red, n_red, p->d_pm, Y, ldy, nr, st);
     HMVM_CUDA_TRY(cudaGetLastError(), "multi-RHS row-stage reduction launch");
   }
   if (ev) cudaEventRecord(ev[4], st);
@@ -1213,13 +1215,13 @@ int tcw_kernels_per_pass(const hmvm_plan* p) {
   return (p->tcw_bf ? 1 : 2) + (p->stage1_tiles > 0) + (p->n_red1 > 0) + 1;
 }
 
-// Right-hand sides per pass, of 8, 4 and 2.  FP64 plans: the narrowest width up
+// Right-hand sides per pass, of 8, 4 and 2.  Plain plans: the narrowest width up
 // to nrhs_max that takes all that is left, else the widest, since a pass costs
 // about the same at every width (the matrix stream).  Others: the widest up to
 // nrhs_max that is not above what is left (a last single column runs in a
 // 2-wide pass).
 int multi_pass_width(const hmvm_plan* p, int left) {
-  if (plan_mode(p) == kModePlain64)
+  if (!p->mixed)
     for (int w : {2, 4, 8})
       if (w <= p->nrhs_max && w >= left) return w;
   for (int w : {8, 4, 2})
@@ -1236,7 +1238,7 @@ std::vector<Pass> multi_passes(const hmvm_plan* p, int nrhs) {
   for (int r0 = 0; r0 < nrhs;) {
     const int w = p->tcw ? kTcwRhs : p->nrhs_max <= 1 ? 1 : p->tc ? kTcNrhs : multi_pass_width(p, nrhs - r0);
     const int nr = std::min(w, nrhs - r0);
-    v.push_back(Pass{r0, nr, w});
+    v.push_back(Pass{r0, nr, p->nrhs_max <= 1 || p->tcw || p->tc ? w : multi_inst_width(p->precision, w)});
     r0 += nr;
   }
   return v;
@@ -1639,7 +1641,10 @@ int hmvm_b200_plan_multi_kernel_count(const hmvm_plan* p, int32_t nrhs) {
     return (nrhs + kTcNrhs - 1) / kTcNrhs * (5 + (p->stage1_tiles > 0) + (p->n_red1 > 0) + 1 + (p->n_red2 > 0));
   int passes = 0;
   for (int r0 = 0; r0 < nrhs; passes++) r0 += std::min(multi_pass_width(p, nrhs - r0), nrhs - r0);
-  return passes * (1 + (p->stage1_tiles > 0) + (p->n_red1 > 0) + 1 + (p->n_red2 > 0));
+  int n1 = 0, n2 = 0;
+  multi_red(p, true, &n1);
+  multi_red(p, false, &n2);
+  return passes * (1 + (p->stage1_tiles > 0) + (n1 > 0) + 1 + (n2 > 0));
 }
 
 static int one_shot(hmvm_plan* plan, const void* x, void* y, hmvm_stats* stats, double setup_s) {
@@ -2113,7 +2118,7 @@ int batch_mode(const hmvm_batch* b) { return plan_mode(b->cls.front().plan); }
 
 template <int MODE, bool VST>
 const void* batch_stage_kernel() {
-  constexpr MultiCfg c = MODE == kModePlain64 ? kDmmaCfg : kMultiCfgs[kDefaultMultiCfg];
+  constexpr MultiCfg c = MODE <= kModePlain32 ? kDmmaCfg : kMultiCfgs[kDefaultMultiCfg];
   return (const void*)hmvm_batch_multi_kernel<c.wpb, c.slots, c.chunk, MODE, VST>;
 }
 const void* batch_stage_kernel_for(int mode, bool vst) {
@@ -2166,7 +2171,7 @@ int batch_create(const std::vector<LeafTable>& tabs, bool is_float, const hmvm_p
   double wsum = 0;
   for (int key : order) {
     BatchClass c;
-    c.width = key / 1024;
+    c.width = multi_inst_width(o.precision, key / 1024);
     c.npass = key % 1024;
     double el = 0;
     for (int32_t m = 0; m < count; m++) {
@@ -2218,9 +2223,7 @@ MultiArgs part_args(const hmvm_plan* p, const PassBufs& q, bool vst, int64_t ldy
   a.pcap = (int64_t)(p->p_len + 16) * w;
   a.ycap = (int64_t)(p->nd + 16) * w;
   a.err = p->d_err;
-  a.tiles = p->d_tiles;
-  a.segs = p->d_segs;
-  multi_teams(p, vst, a);
+  multi_items(p, vst, a);
   a.data = p->d_data;
   a.x64 = q.xm64;
   a.x32 = q.xm32;
@@ -2231,7 +2234,6 @@ MultiArgs part_args(const hmvm_plan* p, const PassBufs& q, bool vst, int64_t ldy
   a.p = q.pm;
   a.out_idx = p->d_out_idx;
   a.scale = p->d_scale;
-  a.seg_first = p->d_segfirst;
   return a;
 }
 
@@ -2303,8 +2305,10 @@ int batch_set_io(hmvm_batch* b, const void* const* X, const int64_t* ldx, void* 
       const PassBufs& pb = c.pass[q];
       if (p->stage1_tiles > 0) stage_add(p1, part_args(p, pb, true, c.ntot), c.width);
       stage_add(p2, part_args(p, pb, false, c.ntot), c.width);
-      red_add(r1, (const int4*)p->d_red1, p->n_red1, pb.pm, pcap, pb.tm, tcap, 0, c.width);
-      red_add(r2, (const int4*)p->d_red2, p->n_red2, pb.pm, pcap, pb.ycat, xcap, c.ntot, c.width);
+      int nred1 = 0, nred2 = 0;
+      const int4 *red1 = multi_red(p, true, &nred1), *red2 = multi_red(p, false, &nred2);
+      red_add(r1, red1, nred1, pb.pm, pcap, pb.tm, tcap, 0, c.width);
+      red_add(r2, red2, nred2, pb.pm, pcap, pb.ycat, xcap, c.ntot, c.width);
       for (size_t i = 0; i < c.members.size(); i++) {
         const int32_t m = c.members[i];
         if (io[m].n == 0 || io[m].nrhs <= q * c.width) continue;  // no columns in this pass

@@ -75,18 +75,15 @@ struct BatchPart {
 };
 template <int WPB, int S, int CHUNK, int MODE, bool VST>
 __global__ void __launch_bounds__(
-    32 * WPB, (MODE == kModePlain64 ? dmma_min_blocks<WPB, S, CHUNK>() : multi_min_blocks<WPB, S, CHUNK, kMultiZBytes>()))
+    32 * WPB, (MODE <= kModePlain32 ? dmma_min_blocks<WPB, S, CHUNK>() : multi_min_blocks<WPB, S, CHUNK, kMultiZBytes>()))
     hmvm_batch_multi_kernel(const BatchPart* __restrict__ parts, int nparts) {
   int k = 0;
   while (k + 1 < nparts && (int)blockIdx.x >= parts[k + 1].cta0) k++;
   const MultiArgs a = parts[k].a;
   const int bid = (int)blockIdx.x - parts[k].cta0;
-  if constexpr (MODE == kModePlain64) {
-    switch (parts[k].nr) {
-      case 2: dmma_body<double, WPB, S, CHUNK, 2, VST, true>(a, bid); break;
-      case 4: dmma_body<double, WPB, S, CHUNK, 4, VST, true>(a, bid); break;
-      default: dmma_body<double, WPB, S, CHUNK, 8, VST, true>(a, bid); break;
-    }
+  if constexpr (MODE <= kModePlain32) {
+    using T = typename std::conditional<MODE == kModePlain64, double, float>::type;
+    dmma_body<T, WPB, S, CHUNK, 0, VST, true>(a, bid, parts[k].nr);
   } else {
     switch (parts[k].nr) {
       case 2: multi_body<WPB, S, CHUNK, 2, MODE, VST, true>(a, bid); break;

@@ -22,8 +22,20 @@
 // against the 23 that HBM delivers, at any NR, so the stream stays the bound.
 // What is left is latency per item (inputs, descriptors, outputs) that 12 warps
 // per SM do not hide.
-// N = 65,536 FP64 sphere (1.04 GB), 8 right-hand sides: V stage 147 -> 76 us
-// (4.8 TB/s), row stage 295 -> 133 us (5.1 TB/s).
+//
+// FP32 plans: the matrix values come from ldmatrix in the operand's layout and
+// are widened to FP64 in registers, as are the inputs, so products and sums are
+// FP64 (error against FP64 2e-7 -> 4e-8).  4 matrix and 1 conversion instruction
+// per vector more than FP64's half vector: the FP64 pipe is busy for half of the
+// row stage.  tf32 or 16-bit splits on the tensor cores would have been less
+// exact than the FP32 sums they replaced.
+//
+// A team adds up the consecutive parts of a tile that it has (one page of inputs
+// each), so only tiles that two teams share have partial sums.
+//
+// Measured, 8 right-hand sides, whole apply (V stage, row stage): N = 65,536 FP64
+// sphere, 1.04 GB: 464 us (147, 295) -> 229 (77, 128: 5.3 TB/s); N = 100,003 FP32
+// cube, 0.95 GB: 401 us (133, 237) -> 256 (86, 155).
 #pragma once
 
 #include "kernels_multi.cuh"
@@ -62,23 +74,28 @@ constexpr int dmma_min_blocks() {
 // The body of hmvm_dmma_kernel for block bid of the launch (a batch launch runs
 // several plans' bodies, each over its own range of blocks).  CHECK: every
 // input range and output row is checked against the buffers' lengths; a miss
-// records error 3 and is skipped.
-template <typename T, int WPB, int S, int CHUNK, int NR, bool VST, bool CHECK = false>
-__device__ __forceinline__ void dmma_body(const MultiArgs& a, int bid) {
+// records error 3 and is skipped.  NRC: the pass width, or 0 for one that is only
+// known at run time (nr; a batch's parts differ, and one body per width made its
+// kernel outgrow the instruction cache: 6 of 11 cycles per instruction waiting
+// for it).
+template <typename T, int WPB, int S, int CHUNK, int NRC, bool VST, bool CHECK = false>
+__device__ __forceinline__ void dmma_body(const MultiArgs& a, int bid, int nr = NRC) {
   constexpr uint32_t RING = (uint32_t)S * CHUNK;
   constexpr uint32_t RSTRIDE = RING + kDmmaRingPad;  // the ring and the copy of its first bytes
   constexpr int VN = 16 / (int)sizeof(T);  // columns per 16-byte vector
   constexpr int SV = 4 / VN;               // vectors per step of 4 columns
   constexpr int B = 8;                     // vectors per batch
   constexpr int NS = B / SV;               // steps per batch
-  constexpr int ES = NR * (int)sizeof(T);  // input bytes per column
-  constexpr int PV = kDmmaPageBytes / (ES * VN);  // vectors per page of inputs
+  const int NR = NRC > 0 ? NRC : nr;       // 2 (FP64 only), 4 or 8
+  const int ES = NR * (int)sizeof(T);      // input bytes per column
+  const int PVL = (NR == 2 ? 3 : NR == 4 ? 2 : 1) + 4;  // log2 of the vectors per page of inputs
+  const int PV = 1 << PVL;
   using T2 = typename std::conditional<std::is_same<T, double>::value, double2, float2>::type;
   static_assert((RING & (RING - 1)) == 0, "ring size must be a power of two");
   static_assert(CHUNK % 16 == 0 && CHUNK >= 512, "bulk copies move multiples of 16 bytes");
   static_assert(B * 32 * 16 <= (S - 1) * CHUNK, "ring too small for one batch");
-  static_assert(NR == 2 || NR == 4 || NR == 8, "one block of 8 result columns");
-  static_assert(PV % B == 0, "batches end with their page");
+  static_assert(NRC == 0 || NRC == 2 || NRC == 4 || NRC == 8, "one block of 8 result columns");
+  static_assert(kDmmaPageBytes == 4096, "pages of 4096 / (16 NR) vectors, a whole number of batches");
   extern __shared__ __align__(128) unsigned char smem[];
 
   const int lane = threadIdx.x & 31;
@@ -167,7 +184,6 @@ __device__ __forceinline__ void dmma_body(const MultiArgs& a, int bid) {
       unsigned char* dst = zb + (p0 - lo) * ES;
       if (copied > 0) bulk_g2s(dst, (from_t ? static_cast<const T*>(a.t) : xin) + src, (uint32_t)(copied * ES), zbar);
       for (int z = copied; z < p1 - p0; z++)
-#pragma unroll
         for (int r = 0; r < ES; r += 16) *reinterpret_cast<uint4*>(dst + z * ES + r) = make_uint4(0, 0, 0, 0);
     }
     if (lane == 0) mbar_arrive(zbar);
@@ -206,7 +222,11 @@ __device__ __forceinline__ void dmma_body(const MultiArgs& a, int bid) {
     // kq / 2; FP32: the 16-byte row that the lane addresses for ldmatrix)
     const uint32_t lane_vec = sizeof(T) == 8 ? (uint32_t)(kq >> 1) * rstride : 0u;
     const unsigned char* lane_ring = ring + (sizeof(T) == 8 ? nq * 16 + (kq & 1) * 8 : lane * 16);
-    double acc[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+    // Sums of the page and of the item: pages are added up in order, which keeps
+    // the chains of additions short.
+    double acc[4][2], sum[4][2];
+#pragma unroll
+    for (int rb = 0; rb < 4; rb++) acc[rb][0] = acc[rb][1] = sum[rb][0] = sum[rb][1] = 0.0;
     // Vectors [v0, v1) of the item, NRB blocks of 8 rows.  Rows past R of the
     // last block read ring bytes of other rows (always inside the ring); a row
     // of the matrix operand only reaches its own row of the result, which is
@@ -273,7 +293,7 @@ __device__ __forceinline__ void dmma_body(const MultiArgs& a, int bid) {
       }
       return true;
     };
-    const int npg = max(1, (nvt + PV - 1) / PV);
+    const int npg = max(1, (nvt + PV - 1) >> PVL);
     for (int pg = 0; pg < npg; pg++, kp++) {
       __syncwarp();  // every lane is done with the page the next gather overwrites
       const uint32_t nbuf = (kp + 1) & 1;
@@ -302,6 +322,13 @@ __device__ __forceinline__ void dmma_body(const MultiArgs& a, int bid) {
         failed = true;
         break;
       }
+#pragma unroll
+      for (int rb = 0; rb < 4; rb++)
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          sum[rb][i] += acc[rb][i];
+          acc[rb][i] = 0.0;
+        }
     }
     if (failed) break;
     uint32_t row_ok = 0xffffffffu;  // rows whose outputs lie inside their buffer
@@ -320,8 +347,8 @@ __device__ __forceinline__ void dmma_body(const MultiArgs& a, int bid) {
       const int slot = VST ? __shfl_sync(0xffffffffu, cur_oidx, row) : 0;
       if (row < R && r < NR && (!CHECK || (row_ok >> row & 1))) {
         T2 val;
-        val.x = (T)acc[rb][0];
-        val.y = (T)acc[rb][1];
+        val.x = (T)sum[rb][0];
+        val.y = (T)sum[rb][1];
         if (VST && cur.mode == 1) {
           *reinterpret_cast<T2*>(static_cast<T*>(a.t) + (int64_t)slot * NR + r) = val;
         } else if (!VST && cur.mode == 0) {

@@ -6,7 +6,8 @@
 //                           row-interleaved input xpk[i * NR + r] (FP64 and/or
 //                           FP32 copies, zero rows past N), so that every
 //                           segment's inputs are one contiguous block.
-//   hmvm_multi_kernel       one warp per team, lane = row; the matrix streams
+//   hmvm_multi_kernel       mixed plans (plain plans: kernels_dmma.cuh): one
+//                           warp per team, lane = row; the matrix streams
 //                           through the warp's TMA ring exactly as in the
 //                           single-vector kernels; each stored element is
 //                           multiplied by its column's NR inputs.  V stage:
@@ -16,12 +17,10 @@
 //                           order, per right-hand side.
 //
 // MODE: kModePlain64 (FP64 plan), kModePlain32 (FP32 plan), kModeMixed16 /
-// kModeMixedBF16 (mixed plan with FP16 / BF16 factors).  Element types per
-// segment follow the plan: FP64 plans store FP64 only, FP32 plans FP32 only,
-// mixed plans carry the type in the segment descriptor.  Inputs: FP64
-// segments read the FP64 copy of x (or the FP64 t of FP64 plans), all others
-// FP32 values.  Sums: FP32 per run of same-type segments (FP64 for FP64
-// segments), FP64 per row.
+// kModeMixedBF16 (mixed plan with FP16 / BF16 factors).  Mixed segments carry
+// their element type in the descriptor; FP64 segments read the FP64 copy of x,
+// all others FP32 values.  Sums: FP32 per run of same-type segments (FP64 for
+// FP64 segments), FP64 per row.
 #pragma once
 
 #include "kernels.cuh"
@@ -85,27 +84,26 @@ __global__ void hmvm_reduce_multi_kernel(const int4* __restrict__ red, int n, co
   }
 }
 
+// Element types of a mixed plan's pass: t FP32, y and the partial sums FP64.
 template <int MODE>
 struct MultiMode {
-  static constexpr bool mixed = MODE >= kModeMixed16;
+  static_assert(MODE >= kModeMixed16, "plain plans run hmvm_dmma_kernel");
   static constexpr int lr16 = MODE == kModeMixedBF16 ? kBF16 : kF16;
-  using TT = typename std::conditional<MODE == kModePlain64, double, float>::type;  // t element
-  using TY = typename std::conditional<MODE == kModePlain32, float, double>::type;  // y / p element
+  using TT = float;
+  using TY = double;
 };
 
 // Copy the inputs item `d` reads into zb: for each segment, ncp columns of
 // NR values (ncp = columns rounded up to whole vectors; the padding is zero).
 // FP64 segments take 8-byte values, the others 4-byte values.
-template <int MODE, int NR, bool CHECK = false>
+template <int NR, bool CHECK = false>
 __device__ __forceinline__ void gather_multi(const hmvm_tile_desc& d, const hmvm_seg_desc& sreg, const MultiArgs& a,
                                              unsigned char* zb, int lane) {
-  using TT = typename MultiMode<MODE>::TT;
   int zoff = 0;
   for (int j = 0; j < d.nseg; j++) {
     const int src = __shfl_sync(0xffffffffu, sreg.src, j);
     const int enc = __shfl_sync(0xffffffffu, sreg.ncols, j);
-    const int type = MultiMode<MODE>::mixed ? (enc >> 28) : (MODE == kModePlain64 ? kF64 : kF32);
-    const int nc = MultiMode<MODE>::mixed ? (enc & 0x0fffffff) : enc;
+    const int type = enc >> 28, nc = enc & 0x0fffffff;
     const int lg = mixed_vec_log2(type);
     const int ncp = ((nc + (1 << lg) - 1) >> lg) << lg;
     const bool from_t = src < 0;
@@ -119,7 +117,7 @@ __device__ __forceinline__ void gather_multi(const hmvm_tile_desc& d, const hmvm
       }
     }
     if (type == kF64) {
-      const double* s = from_t ? reinterpret_cast<const double*>(static_cast<const TT*>(a.t)) + base : a.x64 + base;
+      const double* s = a.x64 + base;  // FP64 segments are dense leaves
       double* z = reinterpret_cast<double*>(zb + zoff);
       if constexpr (NR % 2 == 0) {  // 16-byte copies: (src * NR) is even
         for (int c = lane; c < ncp * NR / 2; c += 32) {
@@ -134,7 +132,7 @@ __device__ __forceinline__ void gather_multi(const hmvm_tile_desc& d, const hmvm
       }
       zoff += ncp * NR * 8;
     } else {
-      const float* s = from_t ? reinterpret_cast<const float*>(static_cast<const TT*>(a.t)) + base : a.x32 + base;
+      const float* s = from_t ? static_cast<const float*>(a.t) + base : a.x32 + base;
       float* z = reinterpret_cast<float*>(zb + zoff);
       if constexpr (NR % 4 == 0) {
         for (int c = lane; c < ncp * NR / 4; c += 32) {
@@ -244,7 +242,7 @@ __device__ __forceinline__ void multi_body(const MultiArgs& a, int bid) {
   using TT = typename MM::TT;
   using TYO = typename MM::TY;
   constexpr uint32_t RING = (uint32_t)S * CHUNK;
-  constexpr int ZB = MODE == kModePlain64 ? kMultiZBytesF64 : kMultiZBytes;  // each of the two input buffers
+  constexpr int ZB = kMultiZBytes;  // each of the two input buffers
   constexpr int B = 2;  // vectors per batch: each carries 2..16 columns of NR products
   static_assert((RING & (RING - 1)) == 0, "ring size must be a power of two");
   static_assert(CHUNK % 16 == 0 && CHUNK >= 512, "bulk copies move multiples of 16 bytes");
@@ -294,7 +292,7 @@ __device__ __forceinline__ void multi_body(const MultiArgs& a, int bid) {
     for (uint32_t q = 0; q < min((uint32_t)S, nchunks); q++) issue(q);
 
   auto row_scale = [&](const hmvm_tile_desc& d) {
-    if constexpr (VST && MM::mixed) return lane < d.nrows ? a.scale[d._pad + lane] : 1.0;
+    if constexpr (VST) return lane < d.nrows ? a.scale[d._pad + lane] : 1.0;
     else return 1.0;
   };
   auto out_slot = [&](const hmvm_tile_desc& d) {
@@ -302,7 +300,7 @@ __device__ __forceinline__ void multi_body(const MultiArgs& a, int bid) {
     else return 0;
   };
   hmvm_seg_desc cur_seg = lane < cur.nseg ? segs[cur.seg_begin + lane] : szero;
-  gather_multi<MODE, NR, CHECK>(cur, cur_seg, a, zbase, lane);
+  gather_multi<NR, CHECK>(cur, cur_seg, a, zbase, lane);
   cp_async_commit();
   int cur_oidx = out_slot(cur);
   double cur_scale = row_scale(cur);
@@ -314,7 +312,7 @@ __device__ __forceinline__ void multi_body(const MultiArgs& a, int bid) {
   for (int ti = tb, k = 0; ti < te; ++ti, ++k) {
     unsigned char* zcur = zbase + (k & 1) * ZB;
     __syncwarp();
-    if (ti + 1 < te) gather_multi<MODE, NR, CHECK>(nxt, nxt_seg, a, zbase + ((k + 1) & 1) * ZB, lane);
+    if (ti + 1 < te) gather_multi<NR, CHECK>(nxt, nxt_seg, a, zbase + ((k + 1) & 1) * ZB, lane);
     cp_async_commit();
     const bool has_nn = ti + 2 < te;
     const hmvm_tile_desc nn = has_nn ? tiles[ti + 2] : dzero;
@@ -379,7 +377,7 @@ __device__ __forceinline__ void multi_body(const MultiArgs& a, int bid) {
     int j = 0;
     while (j < (VST ? 1 : cur.nseg)) {
       const int enc0 = __shfl_sync(0xffffffffu, cur_seg.ncols, j);
-      const int type = MM::mixed ? (enc0 >> 28) : (MODE == kModePlain64 ? kF64 : kF32);
+      const int type = enc0 >> 28;
       const int lg = mixed_vec_log2(type);
       const unsigned char* zs = zcur + zoff;
       int nv = 0;
@@ -389,23 +387,17 @@ __device__ __forceinline__ void multi_body(const MultiArgs& a, int bid) {
       } else {
         for (; j < cur.nseg; j++) {
           const int enc = __shfl_sync(0xffffffffu, cur_seg.ncols, j);
-          if (MM::mixed && (enc >> 28) != type) break;
-          nv += ((MM::mixed ? (enc & 0x0fffffff) : enc) + (1 << lg) - 1) >> lg;
+          if ((enc >> 28) != type) break;
+          nv += ((enc & 0x0fffffff) + (1 << lg) - 1) >> lg;
         }
       }
       zoff += (nv << lg) * NR * (type == kF64 ? 8 : 4);
       bool ok;
-      if constexpr (MODE == kModePlain64) {
-        ok = run_seg(TypeTag<kF64>{}, zs, nv);
-      } else if constexpr (MODE == kModePlain32) {
-        ok = run_seg(TypeTag<kF32>{}, zs, nv);
-      } else {
-        switch (type) {
-          case kF64: ok = run_seg(TypeTag<kF64>{}, zs, nv); break;
-          case kF32: ok = run_seg(TypeTag<kF32>{}, zs, nv); break;
-          case kE4M3: ok = run_seg(TypeTag<kE4M3>{}, zs, nv); break;
-          default: ok = run_seg(TypeTag<MM::lr16>{}, zs, nv); break;
-        }
+      switch (type) {
+        case kF64: ok = run_seg(TypeTag<kF64>{}, zs, nv); break;
+        case kF32: ok = run_seg(TypeTag<kF32>{}, zs, nv); break;
+        case kE4M3: ok = run_seg(TypeTag<kE4M3>{}, zs, nv); break;
+        default: ok = run_seg(TypeTag<MM::lr16>{}, zs, nv); break;
       }
       if (!ok) {
         failed = true;
@@ -461,8 +453,7 @@ __device__ __forceinline__ void multi_body(const MultiArgs& a, int bid) {
 }
 
 template <int WPB, int S, int CHUNK, int NR, int MODE, bool VST>
-__global__ void __launch_bounds__(
-    32 * WPB, (multi_min_blocks<WPB, S, CHUNK, (MODE == kModePlain64 ? kMultiZBytesF64 : kMultiZBytes)>()))
+__global__ void __launch_bounds__(32 * WPB, (multi_min_blocks<WPB, S, CHUNK, kMultiZBytes>()))
     hmvm_multi_kernel(MultiArgs a) {
   multi_body<WPB, S, CHUNK, NR, MODE, VST>(a, (int)blockIdx.x);
 }

@@ -169,7 +169,6 @@ __global__ void __launch_bounds__(32 * WPB, 1) hmvm_tc_kernel(TcArgs ta) {
   constexpr int B = 2;
   constexpr int LR = MM::lr16;
   constexpr uint32_t IDESC = tc_idesc(MODE == kModeMixedBF16 ? 1 : 0, 128, kTcN);
-  static_assert(MM::mixed, "tensor-core passes serve mixed plans");
   static_assert((RING & (RING - 1)) == 0, "ring size must be a power of two");
   static_assert(B * 32 * 16 <= (S - 1) * CHUNK, "ring too small for one batch");
   constexpr int TMEM_COLS = WPB * kTcN <= 32 ? 32 : WPB * kTcN <= 64 ? 64 : WPB * kTcN <= 128 ? 128 : 256;

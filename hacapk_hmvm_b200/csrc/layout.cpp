@@ -127,6 +127,34 @@ int validate_leaves(const LeafTable &lt, std::string &msg) {
   return HMVM_OK;
 }
 
+std::vector<int32_t> even_ranges(const std::vector<int64_t> &cost, int n) {
+  int64_t lo = 0, hi = 0;
+  for (int64_t c : cost) {
+    lo = std::max(lo, c);
+    hi += c;
+  }
+  lo = std::max(lo, hi / std::max(n, 1));
+  const int32_t count = (int32_t)cost.size();
+  auto cut = [&](int64_t cap, std::vector<int32_t> *out) {  // ranges of at most cap
+    int used = 0;
+    for (int32_t i = 0; i < count; used++) {
+      if (out) out->push_back(i);
+      for (int64_t c = cost[i++]; i < count && c + cost[i] <= cap; i++) c += cost[i];
+    }
+    return used;
+  };
+  while (lo < hi) {
+    const int64_t mid = lo + (hi - lo) / 2;
+    if (cut(mid, nullptr) <= n) hi = mid;
+    else lo = mid + 1;
+  }
+  std::vector<int32_t> out;
+  out.reserve((size_t)n + 1);
+  cut(hi, &out);
+  out.resize((size_t)n + 1, count);
+  return out;
+}
+
 int default_stage_cfg(int precision, int kernel, int stage) {
   if (precision == HMVM_MIXED) return stage == 1 ? kDefaultMixedCfg1 : kDefaultMixedCfg2;
   if (kernel == 0) return stage == 1 ? kDefaultStage1Cfg : kDefaultStage2Cfg;
@@ -466,12 +494,11 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
     L.stage2_teams = L.num_sms * L.ctas2_per_sm *
                      (L.mixed ? kMixedCfgs[L.stage2_cfg].wpb : teams_per_cta(L.kernel, L.stage2_cfg));
     if (nrhs_max > 1) {
-      // teams for the multi-RHS kernel, all resident at once (and no more than
-      // the single-vector kernels launch)
-      const bool f64 = !L.mixed && L.elem_size == 8;
-      const int per_sm = nrhs_max == kTcNrhs ? kTcWarpsPerSm : (f64 ? kMultiWarpsPerSmF64 : kMultiWarpsPerSm);
-      L.stage1_teams = std::min(L.stage1_teams, L.num_sms * per_sm);
-      L.stage2_teams = std::min(L.stage2_teams, L.num_sms * per_sm);
+      // teams for the multi-RHS kernel, all resident at once (mixed plans: no more than
+      // the single-vector kernels launch; plain plans give those their own ranges)
+      const int per_sm = nrhs_max == kTcNrhs ? kTcWarpsPerSm : kMultiWarpsPerSm;
+      L.stage1_teams = L.mixed ? std::min(L.stage1_teams, L.num_sms * per_sm) : L.num_sms * kDmmaWarpsPerSm;
+      L.stage2_teams = L.mixed ? std::min(L.stage2_teams, L.num_sms * per_sm) : L.num_sms * kDmmaWarpsPerSm;
     }
     int64_t stage_bytes[2] = {0, 0};
     for (int32_t k = 0; k < ntb; k++) stage_bytes[k < n1 ? 0 : 1] += (int64_t)tb[k].nvec * tb[k].nrows * 16;
@@ -490,6 +517,7 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
     items.reserve((size_t)ntb + ntb / 2);
     std::vector<int32_t> tile_item0(ntb + 1);
     int64_t p_len = 0;
+    const bool runs = !L.mixed && nrhs_max > 1;
     for (int32_t k = 0; k < ntb; k++) {
       const TileBuild &t = tb[k];
       tile_item0[k] = (int32_t)items.size();
@@ -591,6 +619,21 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
                       std::vector<int32_t> &team_begin) {
       std::vector<int32_t> idx(count);
       for (int32_t k = 0; k < count; k++) idx[k] = first + k;
+      if (runs) {
+        // Plain multi-RHS plans: the items stay in order and are cut into ranges
+        // of about the same cost, so that a team adds up the parts of a tile that
+        // it gets.  A vector, a part (a page of inputs) and a tile cost something on
+        // top of the bytes.
+        std::vector<int64_t> cost(count);
+        for (int32_t k = 0; k < count; k++) {
+          const Item &it = items[first + k];
+          cost[k] = (int64_t)(it.vb - it.va) * 16 * (tb[it.tile].nrows + kDmmaStepRows) + kDmmaPartCost +
+                    (it.va == 0 ? kDmmaTileCost : 0);
+        }
+        order = idx;
+        team_begin = even_ranges(cost, nteams);
+        return;
+      }
       std::stable_sort(idx.begin(), idx.end(), [&](int32_t a, int32_t b) { return items[a].cost > items[b].cost; });
       using HE = std::pair<int64_t, int32_t>;
       std::priority_queue<HE, std::vector<HE>, std::greater<HE>> heap;
@@ -658,6 +701,70 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
       d.nseg = nseg;
       item_off[order[k]] = off;
       off += (int64_t)d.nvec * t.nrows;
+    }
+    if (runs) {
+      // The items as hmvm_dmma_kernel runs them: a run is the consecutive parts of
+      // one tile within one team.  A tile of one run needs no partial sums; the
+      // others' runs write theirs at their first part's place.
+      for (int st = 0; st < 2; st++) {
+        const std::vector<int32_t> &tbeg = st == 0 ? L.team_begin1 : L.team_begin2;
+        std::vector<int32_t> &mbeg = st == 0 ? L.mteam_begin1 : L.mteam_begin2;
+        std::vector<int32_t> &red = st == 0 ? L.mred1 : L.mred2;
+        int32_t tile = -1, nruns = 0;  // the tile of the last run and its runs so far
+        auto close = [&]() {
+          if (nruns < 2) return;
+          const TileBuild &t = tb[tile];
+          for (int32_t r = 0; r < t.nrows; r++) {
+            red.push_back(st == 0 ? L.out_idx[t.panel_row0 + r] : t.row0 + r);
+            red.push_back(items[tile_item0[tile]].out_base + r);
+            red.push_back(nruns);
+            red.push_back(t.nrows);
+          }
+        };
+        for (size_t team = 0; team + 1 < tbeg.size(); team++) {
+          mbeg.push_back((int32_t)L.mtiles.size());
+          for (int32_t k = tbeg[team]; k < tbeg[team + 1];) {
+            const TileBuild &t = tb[items[k].tile];
+            const int32_t i0 = tile_item0[items[k].tile], i1 = tile_item0[items[k].tile + 1];
+            const int32_t end = std::min(tbeg[team + 1], i1);
+            if (items[k].tile != tile) {
+              close();
+              tile = items[k].tile;
+              nruns = 0;
+            }
+            hmvm_tile_desc d = L.tiles[k];
+            if (k == i0 && end == i1) {
+              d.mode = (int16_t)t.mode;
+              d.out_base = t.out_base;
+            } else {
+              d.out_base = items[i0].out_base + nruns * t.nrows;  // at most one run per part
+            }
+            nruns++;
+            d.seg_begin = (int32_t)L.msegs.size();
+            d.nvec = 0;
+            int32_t col = 0;
+            for (; k < end; k++) {
+              const hmvm_tile_desc &part = L.tiles[k];
+              d.nvec += part.nvec;
+              for (int32_t s = part.seg_begin; s < part.seg_begin + part.nseg; s++) {
+                const hmvm_seg_desc &sg = L.segs[s];
+                hmvm_seg_desc *last = (int32_t)L.msegs.size() > d.seg_begin ? &L.msegs.back() : nullptr;
+                if (s == part.seg_begin && last && last->ncols % VEC == 0 && last->src + last->ncols == sg.src) {
+                  last->ncols += sg.ncols;  // a segment that the cut between two parts went through
+                } else {
+                  L.msegs.push_back(sg);
+                  L.mseg_first.push_back(col);
+                }
+                col += (sg.ncols + VEC - 1) / VEC * VEC;
+              }
+            }
+            d.nseg = (int32_t)L.msegs.size() - d.seg_begin;
+            L.mtiles.push_back(d);
+          }
+        }
+        close();
+        mbeg.push_back((int32_t)L.mtiles.size());
+      }
     }
     // Not zeroed (UninitAlloc): the items partition [0, off) and the pack
     // below copies every item's whole range from a zero-padded tile buffer.

@@ -164,11 +164,11 @@ constexpr int kDefaultMixedCfg2 = 8;
 constexpr int kMaxNrhsPass = 8;   // CUDA-core multi-RHS passes
 constexpr int kTcNrhs = 16;        // tensor-core passes (mixed plans with nrhs_max = 16)
 constexpr int kTcWarpsPerSm = 7;   // resident warps (teams) per SM of the tensor-core kernel
-// Each warp's two input buffers of the multi-RHS kernel (an item's x/t columns
-// for all of a pass's right-hand sides): 4 KiB each lets 3 CTAs of 4 warps
-// share an SM (12 warps; 8 with 8 KiB: 12 % faster at 8 FP32 right-hand sides).
-// FP64 plans keep 8 KiB and 8 warps: their inputs are twice as wide, and 4 KiB
-// cut their items twice as often (10 % slower at 8 right-hand sides).
+// Each warp's two input buffers of hmvm_multi_kernel (an item's x/t columns for
+// all of a pass's right-hand sides): 4 KiB each lets 3 CTAs of 4 warps share an
+// SM (12 warps; 8 with 8 KiB: 12 % slower at 8 right-hand sides).  Plain plans'
+// items keep to the same bounds (FP64 8 KiB), though hmvm_dmma_kernel reads its
+// inputs in pages: they are the parts that its warps are given.
 constexpr int kMultiZBytes = 4096;
 constexpr int kMultiZBytesF64 = 8192;
 constexpr int multi_zbytes(bool f64) { return f64 ? kMultiZBytesF64 : kMultiZBytes; }
@@ -181,28 +181,29 @@ struct MultiCfg {
 // 4 x 2 KiB and 8 x 1 KiB rings it replaced)
 constexpr int kNumMultiCfgs = 1;
 constexpr MultiCfg kMultiCfgs[kNumMultiCfgs] = {{4, 2, 4096}};
-inline int multi_smem_bytes(const MultiCfg& c, bool f64) {
-  return c.wpb * (c.slots * c.chunk + 2 * multi_zbytes(f64) + c.slots * 8);
-}
+inline int multi_smem_bytes(const MultiCfg& c) { return c.wpb * (c.slots * c.chunk + 2 * kMultiZBytes + c.slots * 8); }
 constexpr int kDefaultMultiCfg = 0;
 // hmvm_dmma_kernel: 3 CTAs of 4 warps per SM; per warp a ring of 2 x 4 KiB, the
 // copy of its first bytes (one vector of 32 rows) and two pages of inputs.  At
-// N = 65,536 FP64 with 8 right-hand sides, both stages: 12 warps 209 us; 8 warps
-// with rings of 2 x 8 KiB 212; 16 warps with pages of 2 KiB 214; 12 warps with
-// rings of 4 x 2 KiB 242 (every bulk copy costs the TMA unit some 20 cycles);
-// without the L2 prefetch of the next chunk 241.
+// N = 65,536 FP64 with 8 right-hand sides, both stages (before the parts of a
+// tile were added up in the kernel): 12 warps 209 us; 8 warps with rings of
+// 2 x 8 KiB 212; 16 warps with pages of 2 KiB 214; 12 warps with rings of
+// 4 x 2 KiB 242 (every bulk copy costs the TMA unit some 20 cycles); without the
+// L2 prefetch of the next chunk 241.
 constexpr MultiCfg kDmmaCfg = {4, 2, 4096};
 constexpr int kDmmaPageBytes = 4096;
 constexpr int kDmmaRingPad = 512;
 constexpr int kDmmaWarpsPerSm = 12;
-// An item's fixed cost in bytes when the kernel's warps are given their items
-// (1.1 us per item against 6 us for the 21 KB of an average one).
-constexpr int64_t kDmmaItemOverhead = 4096;
+// Cost of an item's part in bytes when its teams get their ranges: its vectors of
+// nrows + kDmmaStepRows rows, kDmmaPartCost, and kDmmaTileCost for a tile's first
+// part.  V stage of 8 FP32 right-hand sides (N = 100,003): 86 us; with 4 KiB less
+// per tile 105, with 8 KiB more 95, without the rows' share 112.
+constexpr int kDmmaStepRows = 8;
+constexpr int64_t kDmmaPartCost = 2048, kDmmaTileCost = 4096;
 constexpr int dmma_smem_bytes(const MultiCfg& c) {
   return c.wpb * (c.slots * c.chunk + kDmmaRingPad + 2 * kDmmaPageBytes + (c.slots + 2) * 8);
 }
 constexpr int kMultiWarpsPerSm = 12;    // resident warps (teams) per SM of the multi-RHS kernel
-constexpr int kMultiWarpsPerSmF64 = 8;  // the same for FP64 plans (8 KiB input buffers)
 
 // Wide tensor-core passes (plans with nrhs_max >= kTcwMinNrhs, FP32 or mixed
 // storage): 128 right-hand sides per pass, every product on tcgen05.
@@ -270,6 +271,14 @@ struct HostLayout {
   int64_t stored_bytes = 0;      // bytes of the stored elements in their storage formats
   int64_t stored_bytes1 = 0;     // ... of the V stage
   int nrhs_max = 1;              // items fit the multi-RHS input buffer for this many rhs
+  // plain plans with nrhs_max > 1: the items as hmvm_dmma_kernel runs them, each
+  // all the parts of a tile that a team has (its inputs come in pages, so they are
+  // not bounded by a buffer), over the same data stream
+  std::vector<hmvm_tile_desc> mtiles;
+  std::vector<hmvm_seg_desc> msegs;
+  std::vector<int32_t> mseg_first;             // per segment: its first padded column within its item
+  std::vector<int32_t> mteam_begin1, mteam_begin2;  // absolute indices into mtiles
+  std::vector<int32_t> mred1, mred2;           // as red1, red2
   // wide tensor-core layout
   bool tcw = false;
   bool tcw_bf16 = false;          // 16-bit format of the stored pairs and the input planes
@@ -288,6 +297,10 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
                  std::string &msg, int ctas2_per_sm = 0);
 
 int validate_leaves(const LeafTable &lt, std::string &msg);
+
+// Items of these costs, in order, cut into n ranges whose largest cost is as
+// small as whole items allow: n + 1 bounds (the last ranges may be empty).
+std::vector<int32_t> even_ranges(const std::vector<int64_t> &cost, int n);
 
 // The wide tensor-core layout (see layout_tc.cpp).
 int build_tc_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, HostLayout &out,

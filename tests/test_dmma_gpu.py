@@ -2,7 +2,7 @@
 edges of its tiles: blocks of 8 rows, steps of 4 columns, batches of 8 vectors,
 pages of inputs, groups of 32 segments, pass widths 2 / 4 / 8 with ragged last
 passes.  Against the FP64 oracle per column; the bars are those of the
-single-vector kernels (FP64 1e-12).
+single-vector kernels (FP64 1e-12, FP32 1e-5).
 """
 import numpy as np
 import pytest
@@ -12,8 +12,8 @@ from helpers import oracle_hmvm, relerr
 
 pytestmark = pytest.mark.gpu
 
-TOL = {"fp64": 1e-12}
-PRECISIONS = ["fp64"]
+TOL = {"fp64": 1e-12, "fp32": 1e-5}
+PRECISIONS = ["fp64", "fp32"]
 
 
 def _apply(plan, X):
