@@ -25,6 +25,7 @@ namespace hmvm {
 
 thread_local std::string g_last_error;
 
+int solve_workspace(hmvm_plan* plan, size_t bytes, void** dev, bool* kept);
 int set_error(int status, const std::string& msg) {
   g_last_error = msg;
   return status;
@@ -248,6 +249,8 @@ struct hmvm_plan {
   size_t xh_bytes = 0;
   cudaStream_t cs_in = nullptr, cs_out = nullptr;  // apply_multi_host: copy streams
   std::vector<cudaEvent_t> pass_events;            // apply_multi_host: per-pass ordering
+  void* d_ws = nullptr;  // solvers' work vectors, kept from the first solve on (up to kKeptWorkspace)
+  size_t ws_bytes = 0;
   // profiling: kEventsPerApply events per recorded apply
   bool profiling = false;
   cudaGraph_t graph = nullptr;       // hmvm_b200_plan_capture: one apply
@@ -283,7 +286,8 @@ void free_plan_buffers(hmvm_plan* p) {
                   p->d_xplanes, p->d_tplanes, p->d_scal, p->d_amax, p->d_xpl, p->d_tpl,
                   p->d_tscale, p->d_xscale, p->d_amax128, p->d_part, p->d_tblocks, p->d_tgroups,
                   p->d_tops, p->d_tgfirst, p->d_segfirst,
-                  p->d_tbm1, p->d_tbm2, p->d_mtiles, p->d_msegs, p->d_mred1, p->d_mred2};
+                  p->d_tbm1, p->d_tbm2, p->d_mtiles, p->d_msegs, p->d_mred1, p->d_mred2,
+                  p->d_ws};
   for (void* b : bufs)
     if (b) cudaFree(b);
 }
@@ -1330,6 +1334,35 @@ void table_from_leaves64(const hmvm_leaves64* lv, bool is_float, LeafTable& lt) 
 }
 
 }  // namespace
+
+// Work vectors of a solve on `plan`, whose device is current.  Up to
+// kKeptWorkspace bytes stay with the plan (allocating and freeing device memory
+// costs a solve milliseconds) and are released with it; larger ones are the
+// caller's to free.  Solves on one plan share them, as they share its t and
+// partial sums: one at a time.
+constexpr size_t kKeptWorkspace = (size_t)64 << 20;
+int hmvm::solve_workspace(hmvm_plan* plan, size_t bytes, void** dev, bool* kept) {
+  *kept = bytes <= kKeptWorkspace;
+  if (*kept && plan->ws_bytes >= bytes) {
+    *dev = plan->d_ws;
+    return HMVM_OK;
+  }
+  if (*kept) {
+    if (plan->d_ws) cudaFree(plan->d_ws);
+    plan->d_ws = nullptr;
+    plan->ws_bytes = 0;
+  }
+  const cudaError_t e = cudaMalloc(dev, bytes);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return HMVM_ENOMEM;
+  }
+  if (*kept) {
+    plan->d_ws = *dev;
+    plan->ws_bytes = bytes;
+  }
+  return HMVM_OK;
+}
 
 extern "C" {
 

@@ -8,8 +8,14 @@
 // A-orthogonalised against the last m (restarted cyclically).  All vectors
 // stay on the device; the inner products are summed in a fixed order
 // (per-block partial sums, then one block), so a solve is repeatable bit for
-// bit; their values come back to the host for the scalars and the stopping
-// test ||r|| / ||b|| < eps.
+// bit.  BiCGSTAB's scalars stay on the device too: every kernel that needs one
+// adds up the partial sums itself, and the host reads one record per step, for
+// the stopping test ||r|| / ||b|| < eps.  GCR(m) reads its inner products back.
+//
+// BiCGSTAB at N = 12,000 (FP64, 7 steps, 15 products of 45 us): 2.1 to 5.5 ms
+// (the allocator's share varies) with work vectors allocated and freed by each
+// call and three round trips to the host per step, 0.86 ms with the plan's
+// workspace and one.  What is left is the products and the gaps before them.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -20,6 +26,8 @@
 
 namespace hmvm {
 int set_error(int status, const std::string& msg);
+// Device memory of a plan for the length of a solve (hmvm_b200.cu).
+int solve_workspace(hmvm_plan* plan, size_t bytes, void** dev, bool* kept);
 }
 using hmvm::set_error;
 
@@ -162,76 +170,192 @@ struct Solver {
   }
 };
 
+// ---- BiCGSTAB ------------------------------------------------------------------
+// The record that the host reads once per step, and the scalars between kernels.
+struct BicgState {
+  double bb, rr;             // b . b and r . r
+  double alpha, zeta, beta;  // of the last step
+  double nom;                // shadow . r at its start
+  int32_t breakdown;         // 1: shadow . A p vanished (the step was not taken)
+  int32_t _pad;
+};
+
+// The two sums of kDotBlocks partial pairs, in dot2_final's order, for every
+// thread of a block of kDotBlocks threads.
+__device__ __forceinline__ void sum_partials(const double* __restrict__ part, double& a, double& b) {
+  __shared__ double s0[kDotBlocks], s1[kDotBlocks];
+  const int t = threadIdx.x;
+  s0[t] = part[2 * t];
+  s1[t] = part[2 * t + 1];
+  __syncthreads();
+  for (int w = kDotBlocks / 2; w > 0; w >>= 1) {
+    if (t < w) {
+      s0[t] += s0[t + w];
+      s1[t] += s1[t + w];
+    }
+    __syncthreads();
+  }
+  a = s0[0];
+  b = s1[0];
+}
+// The block's sums of every thread's (a, b) into its pair of `part`.
+__device__ __forceinline__ void block_partials(double a, double b, double* __restrict__ part) {
+  __shared__ double s0[kDotThreads], s1[kDotThreads];
+  s0[threadIdx.x] = a;
+  s1[threadIdx.x] = b;
+  __syncthreads();
+  for (int w = kDotThreads / 2; w > 0; w >>= 1) {
+    if (threadIdx.x < w) {
+      s0[threadIdx.x] += s0[threadIdx.x + w];
+      s1[threadIdx.x] += s1[threadIdx.x + w];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = s0[0];
+    part[2 * blockIdx.x + 1] = s1[0];
+  }
+}
+static_assert(kDotBlocks == kDotThreads, "one thread per partial pair");
+
+// r = shadow = b - A u; partial sums of b . b and r . r
+template <typename T>
+__global__ void bicg_start(const T* __restrict__ b, const T* __restrict__ au, T* __restrict__ r, T* __restrict__ sh,
+                           int n, double* __restrict__ part) {
+  double a0 = 0.0, a1 = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double bi = (double)b[i];
+    const T ri = (T)(bi - (double)au[i]);
+    r[i] = ri;
+    sh[i] = ri;
+    a0 += bi * bi;
+    a1 += (double)ri * (double)ri;
+  }
+  block_partials(a0, a1, part);
+}
+// The scalars of the step that ended (first: of the start), then
+// p = r + beta (p - zeta A p)
+template <typename T>
+__global__ void bicg_direction(const T* __restrict__ r, const T* __restrict__ akp, T* __restrict__ p, int n, bool first,
+                               const double* __restrict__ part, const BicgState* __restrict__ in,
+                               BicgState* __restrict__ out) {
+  double d0, d1;
+  sum_partials(part, d0, d1);
+  const BicgState st = first ? BicgState{} : *in;
+  const double beta = first ? 0.0 : st.alpha / st.zeta * d0 / st.nom;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    BicgState o = st;
+    if (first) o.bb = d0;
+    o.rr = d1;
+    o.beta = beta;
+    *out = o;
+  }
+  if (st.breakdown) return;
+  const double bz = -beta * st.zeta;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double v = (double)r[i];
+    if (!first) {
+      v += beta * (double)p[i];
+      v += bz * (double)akp[i];
+    }
+    p[i] = (T)v;
+  }
+}
+// alpha from the partial sums of shadow . r and shadow . A p; t = r - alpha A p
+template <typename T>
+__global__ void bicg_half(const T* __restrict__ r, const T* __restrict__ akp, T* __restrict__ t, int n,
+                          const double* __restrict__ part, BicgState* __restrict__ state) {
+  double nom, den;
+  sum_partials(part, nom, den);
+  const double alpha = den != 0.0 ? nom / den : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    state->nom = nom;
+    state->alpha = alpha;
+    state->breakdown = den == 0.0;
+  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    t[i] = (T)((double)r[i] + -alpha * (double)akp[i]);
+}
+// zeta from the partial sums of A t . t and A t . A t; u += alpha p + zeta t,
+// r = t - zeta A t; partial sums of shadow . r and r . r.  A broken-down step
+// leaves u, r and the sums alone.
+template <typename T>
+__global__ void bicg_step(T* __restrict__ u, T* __restrict__ r, const T* __restrict__ p, const T* __restrict__ t,
+                          const T* __restrict__ akt, const T* __restrict__ sh, int n, const double* __restrict__ part,
+                          BicgState* __restrict__ state, double* __restrict__ part_out) {
+  double znom, zden;
+  sum_partials(part, znom, zden);
+  if (state->breakdown) return;
+  const double alpha = state->alpha, zeta = zden != 0.0 ? znom / zden : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) state->zeta = zeta;
+  double a0 = 0.0, a1 = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double ti = (double)t[i];
+    double v = (double)u[i] + alpha * (double)p[i];
+    v += zeta * ti;
+    u[i] = (T)v;
+    const T ri = (T)(ti + -zeta * (double)akt[i]);
+    r[i] = ri;
+    a0 += (double)sh[i] * (double)ri;
+    a1 += (double)ri * (double)ri;
+  }
+  block_partials(a0, a1, part_out);
+}
+
 template <typename T>
 int bicgstab_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, double eps, int32_t* steps_out,
                double* relres_out, cudaStream_t st) {
-  T* buf = nullptr;
-  double* part = nullptr;
-  // r, shadow, p, t, kp (= p), akp, akt, and a copy slot
-  if (cudaMalloc(&buf, sizeof(T) * (size_t)n * 7) != cudaSuccess ||
-      cudaMalloc(&part, sizeof(double) * (2 * kDotBlocks + 2)) != cudaSuccess) {
-    if (buf) cudaFree(buf);
-    cudaGetLastError();
-    return set_error(HMVM_ENOMEM, "bicgstab: device vectors");
-  }
-  T *r = buf, *sh = buf + n, *p = buf + 2 * (size_t)n, *t = buf + 3 * (size_t)n, *akp = buf + 4 * (size_t)n,
-    *akt = buf + 5 * (size_t)n, *kt = buf + 6 * (size_t)n;
-  Solver<T> s{plan, n, st, part, {0, 0}};
-  int rc = HMVM_OK;
-  double bb = 0, rr = 0, relres = 0;
+  // r, shadow, p, t, A p, A t; three sets of partial sums; two state records
+  const size_t ld = ((size_t)n + 31) / 32 * 32, vec_bytes = 6 * ld * sizeof(T);
+  void* ws = nullptr;
+  bool kept = false;
+  int rc = hmvm::solve_workspace(plan, vec_bytes + 6 * kDotBlocks * sizeof(double) + 2 * sizeof(BicgState), &ws, &kept);
+  if (rc) return set_error(HMVM_ENOMEM, "bicgstab: device vectors");
+  T *r = static_cast<T*>(ws), *sh = r + ld, *p = r + 2 * ld, *t = r + 3 * ld, *akp = r + 4 * ld, *akt = r + 5 * ld;
+  double* part0 = reinterpret_cast<double*>(static_cast<char*>(ws) + vec_bytes);
+  double *part1 = part0 + 2 * kDotBlocks, *part2 = part1 + 2 * kDotBlocks;
+  BicgState* state = reinterpret_cast<BicgState*>(part2 + 2 * kDotBlocks);  // [2], alternating
+  BicgState h{};
+  double bnorm = 0, relres = 0;
   int steps = 0;
-  cudaMemsetAsync(p, 0, sizeof(T) * n, st);
-  cudaMemsetAsync(akp, 0, sizeof(T) * n, st);
-  // r = b - A u; shadow = r
   rc = hmvm_b200_apply(plan, u, akt, st);
-  if (!rc) {
-    s.lin(r, b, -1.0, akt);
-    cudaMemcpyAsync(sh, r, sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
-    rc = s.dot2(b, b, r, r, &bb, &rr);
-  }
-  const double bnorm = std::sqrt(bb);
-  relres = bnorm > 0 ? std::sqrt(rr) / bnorm : 0.0;
-  double alpha = 0, beta = 0, zeta = 0, nom_old = 1;
-  while (!rc && relres >= eps && steps < max_steps) {
-    // p = r + beta (p - zeta akp)
-    s.lin(p, r, beta, p, -beta * zeta, akp);
-    rc = hmvm_b200_apply(plan, p, akp, st);
-    if (rc) break;
-    double nom, den;
-    rc = s.dot2(sh, r, sh, akp, &nom, &den);
-    if (rc) break;
-    if (den == 0.0) {
+  if (!rc) bicg_start<T><<<kDotBlocks, kDotThreads, 0, st>>>(b, akt, r, sh, n, part0);
+  for (int k = 0; !rc; k++) {
+    // the next direction; its record tells how the step before it ended
+    BicgState *in = state + (k & 1 ? 0 : 1), *out = state + (k & 1 ? 1 : 0);
+    bicg_direction<T><<<kDotBlocks, kDotThreads, 0, st>>>(r, akp, p, n, k == 0, part0, in, out);
+    if (cudaMemcpyAsync(&h, out, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess) {
+      rc = set_error(HMVM_ECUDA, "bicgstab: inner products");
+      break;
+    }
+    if (h.breakdown) {
       rc = set_error(HMVM_EINVAL, "bicgstab: breakdown (shadow residual orthogonal to A p)");
       break;
     }
-    alpha = nom / den;
-    nom_old = nom;
-    s.lin(t, r, -alpha, akp);  // t = r - alpha akp
-    cudaMemcpyAsync(kt, t, sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
-    rc = hmvm_b200_apply(plan, kt, akt, st);
-    if (rc) break;
-    double znom, zden;
-    rc = s.dot2(akt, t, akt, akt, &znom, &zden);
-    if (rc) break;
-    zeta = zden != 0.0 ? znom / zden : 0.0;
-    s.lin(u, u, alpha, p, zeta, kt);    // u += alpha p + zeta t
-    s.lin(r, t, -zeta, akt);            // r = t - zeta akt
-    double shr;
-    rc = s.dot2(sh, r, r, r, &shr, &rr);
-    if (rc) break;
-    if (zeta == 0.0 || nom_old == 0.0) {
-      steps++;
-      relres = std::sqrt(rr) / bnorm;
-      rc = set_error(HMVM_EINVAL, "bicgstab: breakdown (zeta or rho vanished)");
-      break;
+    if (k == 0) {
+      bnorm = std::sqrt(h.bb);
+      relres = bnorm > 0 ? std::sqrt(h.rr) / bnorm : 0.0;
+    } else {
+      steps = k;
+      relres = std::sqrt(h.rr) / bnorm;
+      if (h.zeta == 0.0 || h.nom == 0.0) {
+        rc = set_error(HMVM_EINVAL, "bicgstab: breakdown (zeta or rho vanished)");
+        break;
+      }
     }
-    beta = alpha / zeta * shr / nom_old;
-    relres = std::sqrt(rr) / bnorm;
-    steps++;
+    if (!(relres >= eps) || k >= max_steps) break;
+    rc = hmvm_b200_apply(plan, p, akp, st);
+    if (rc) break;
+    dot2_partial<T><<<kDotBlocks, kDotThreads, 0, st>>>(sh, r, sh, akp, n, part1);
+    bicg_half<T><<<kDotBlocks, kDotThreads, 0, st>>>(r, akp, t, n, part1, out);
+    rc = hmvm_b200_apply(plan, t, akt, st);
+    if (rc) break;
+    dot2_partial<T><<<kDotBlocks, kDotThreads, 0, st>>>(akt, t, akt, akt, n, part2);
+    bicg_step<T><<<kDotBlocks, kDotThreads, 0, st>>>(u, r, p, t, akt, sh, n, part2, out, part0);
   }
   cudaStreamSynchronize(st);
-  cudaFree(buf);
-  cudaFree(part);
+  if (!kept) cudaFree(ws);
   if (steps_out) *steps_out = steps;
   if (relres_out) *relres_out = relres;
   if (!rc) rc = hmvm_b200_plan_status(plan);
@@ -241,17 +365,14 @@ int bicgstab_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, double e
 template <typename T>
 int gcrm_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, int m, double eps, int32_t* steps_out,
            double* relres_out, cudaStream_t st) {
-  T* buf = nullptr;
-  double* part = nullptr;
-  // r, ar, then the m directions p and their products ap
-  const size_t ld = (size_t)n;
-  if (cudaMalloc(&buf, sizeof(T) * ld * (2 + 2 * (size_t)m)) != cudaSuccess ||
-      cudaMalloc(&part, sizeof(double) * ((size_t)kDotBlocks * (m + 2) + m + 2)) != cudaSuccess) {
-    if (buf) cudaFree(buf);
-    cudaGetLastError();
+  // r, ar, then the m directions p and their products ap; partial sums and inner products
+  const size_t ld = ((size_t)n + 31) / 32 * 32, vec_bytes = sizeof(T) * ld * (2 + 2 * (size_t)m);
+  void* ws = nullptr;
+  bool kept = false;
+  if (hmvm::solve_workspace(plan, vec_bytes + sizeof(double) * ((size_t)kDotBlocks * (m + 2) + m + 2), &ws, &kept))
     return set_error(HMVM_ENOMEM, "gcrm: device vectors");
-  }
-  T *r = buf, *ar = buf + ld, *p = buf + 2 * ld, *ap = buf + (2 + (size_t)m) * ld;
+  T *r = static_cast<T*>(ws), *ar = r + ld, *p = r + 2 * ld, *ap = r + (2 + (size_t)m) * ld;
+  double* part = reinterpret_cast<double*>(static_cast<char*>(ws) + vec_bytes);
   double* dots = part + (size_t)kDotBlocks * (m + 2);
   Solver<T> s{plan, n, st, part, {0, 0}};
   std::vector<double> capap(m, 0.0), hd(m, 0.0);
@@ -262,7 +383,7 @@ int gcrm_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, int m, doubl
   rc = hmvm_b200_apply(plan, u, ar, st);
   if (!rc) {
     s.lin(r, b, -1.0, ar);
-    cudaMemcpyAsync(p, r, sizeof(T) * ld, cudaMemcpyDeviceToDevice, st);
+    cudaMemcpyAsync(p, r, sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
     rc = s.dot2(b, b, r, r, &bb, &rr);
   }
   const double bnorm = std::sqrt(bb);
@@ -290,8 +411,8 @@ int gcrm_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, int m, doubl
     rc = hmvm_b200_apply(plan, r, ar, st);  // ar = A r
     if (rc) break;
     const int ikn = in % m;
-    cudaMemcpyAsync(p + (size_t)ikn * ld, r, sizeof(T) * ld, cudaMemcpyDeviceToDevice, st);
-    cudaMemcpyAsync(ap + (size_t)ikn * ld, ar, sizeof(T) * ld, cudaMemcpyDeviceToDevice, st);
+    cudaMemcpyAsync(p + (size_t)ikn * ld, r, sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
+    cudaMemcpyAsync(ap + (size_t)ikn * ld, ar, sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
     // beta_il = -(ap_il . ar) / capap_il for il = 0..ik, all against the same ar
     const int k = ik + 1;
     dotm_partial<T><<<dim3(kDotBlocks, k), kDotThreads, 0, st>>>(ap, ld, ar, n, part);
@@ -306,8 +427,7 @@ int gcrm_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, int m, doubl
     gcr_update<T><<<(n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184, 256, 0, st>>>(p, ap, ld, k, ikn, be, n);
   }
   cudaStreamSynchronize(st);
-  cudaFree(buf);
-  cudaFree(part);
+  if (!kept) cudaFree(ws);
   if (steps_out) *steps_out = steps;
   if (relres_out) *relres_out = relres;
   if (!rc) rc = hmvm_b200_plan_status(plan);

@@ -279,7 +279,9 @@ int hmvm_b200_batch_kernel_count(const hmvm_batch *batch);
  * type; two HMVMs (hmvm_b200_apply) per step, inner products summed in a fixed
  * order (repeatable).  *steps and *relres receive the steps taken and the
  * final relative residual.  Returns HMVM_EINVAL on a breakdown (a vanishing
- * BiCGSTAB scalar).  Allocates 7 work vectors for the call. */
+ * BiCGSTAB scalar).  Its 6 work vectors stay with the plan for later solves if
+ * they take at most 64 MiB, else they are allocated for the call; solves on one
+ * plan run one at a time. */
 int hmvm_b200_bicgstab(hmvm_plan *plan, const void *b_dev, void *u_dev, int32_t max_steps, double eps,
                        int32_t *steps, double *relres, void *stream);
 /* Solves H u = b by GCR(m), restating HACApK_gcrm_lfmtx
@@ -287,7 +289,7 @@ int hmvm_b200_bicgstab(hmvm_plan *plan, const void *b_dev, void *u_dev, int32_t 
  * m = param(87) in 1..64, eps = param(91)): one HMVM per step, each new search
  * direction A-orthogonalised against the last `restart` (stored cyclically).
  * Same conventions as hmvm_b200_bicgstab; HMVM_EINVAL on a breakdown (A p = 0).
- * Allocates 2 + 2 * restart work vectors for the call. */
+ * Its 2 + 2 * restart work vectors are kept or allocated likewise. */
 int hmvm_b200_gcrm(hmvm_plan *plan, const void *b_dev, void *u_dev, int32_t max_steps, int32_t restart, double eps,
                    int32_t *steps, double *relres, void *stream);
 
