@@ -306,6 +306,9 @@ __device__ __forceinline__ void multi_body(const MultiArgs& a, int bid) {
   double cur_scale = row_scale(cur);
   hmvm_tile_desc nxt = tb + 1 < te ? tiles[tb + 1] : dzero;
   hmvm_seg_desc nxt_seg = (tb + 1 < te && lane < nxt.nseg) ? segs[nxt.seg_begin + lane] : szero;
+  int nxt_oidx = tb + 1 < te ? out_slot(nxt) : 0;
+  double nxt_scale = tb + 1 < te ? row_scale(nxt) : 1.0;
+  hmvm_tile_desc nn = tb + 2 < te ? tiles[tb + 2] : dzero;
 
   uint32_t q_ready = 0, q_rel = 0;
   bool failed = false;
@@ -314,10 +317,12 @@ __device__ __forceinline__ void multi_body(const MultiArgs& a, int bid) {
     __syncwarp();
     if (ti + 1 < te) gather_multi<NR, CHECK>(nxt, nxt_seg, a, zbase + ((k + 1) & 1) * ZB, lane);
     cp_async_commit();
+    // loads for two items ahead; they land while this item runs
     const bool has_nn = ti + 2 < te;
-    const hmvm_tile_desc nn = has_nn ? tiles[ti + 2] : dzero;
-    const int nxt_oidx = ti + 1 < te ? out_slot(nxt) : 0;
-    const double nxt_scale = ti + 1 < te ? row_scale(nxt) : 1.0;
+    const hmvm_seg_desc nn_seg = (has_nn && lane < nn.nseg) ? segs[nn.seg_begin + lane] : szero;
+    const int nn_oidx = has_nn ? out_slot(nn) : 0;
+    const double nn_scale = has_nn ? row_scale(nn) : 1.0;
+    const hmvm_tile_desc nnn = ti + 3 < te ? tiles[ti + 3] : dzero;
     cp_async_wait<1>();
     __syncwarp();
 
@@ -442,7 +447,10 @@ __device__ __forceinline__ void multi_body(const MultiArgs& a, int bid) {
     cur_oidx = nxt_oidx;
     cur_scale = nxt_scale;
     nxt = nn;
-    nxt_seg = (has_nn && lane < nn.nseg) ? segs[nn.seg_begin + lane] : szero;
+    nxt_seg = nn_seg;
+    nxt_oidx = nn_oidx;
+    nxt_scale = nn_scale;
+    nn = nnn;
   }
   cp_async_wait<0>();
   if (failed) {

@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(32 * WPB, 1) hmvm_tc_kernel(TcArgs ta) {
     double cur_scale = row_scale(cur);
     hmvm_tile_desc nxt = tb + 1 < te ? tiles[tb + 1] : dzero;
     hmvm_seg_desc nxt_seg = (tb + 1 < te && lane < nxt.nseg) ? segs[nxt.seg_begin + lane] : szero;
+    hmvm_tile_desc nn = tb + 2 < te ? tiles[tb + 2] : dzero;
 
     for (int ti = tb, k = 0; ti < te && !failed; ++ti, ++k) {
       unsigned char* zcur = zbase + (k & 1) * kTcZBytes;
@@ -338,8 +339,9 @@ __global__ void __launch_bounds__(32 * WPB, 1) hmvm_tc_kernel(TcArgs ta) {
         gather(nxt, nxt_seg, zbase + ((k + 1) & 1) * kTcZBytes, &zbars[(k + 1) & 1], &nxt_k16);
         zpend[(k + 1) & 1] = true;
       }
-      const bool has_nn = ti + 2 < te;
-      const hmvm_tile_desc nn = has_nn ? tiles[ti + 2] : dzero;
+      // descriptors two items ahead: they land while this item runs
+      const hmvm_seg_desc nn_seg = (ti + 2 < te && lane < nn.nseg) ? segs[nn.seg_begin + lane] : szero;
+      const hmvm_tile_desc nnn = ti + 3 < te ? tiles[ti + 3] : dzero;
       const int nxt_oidx = ti + 1 < te ? out_slot(nxt) : 0;
       const double nxt_scale = ti + 1 < te ? row_scale(nxt) : 1.0;
       if (!warp_wait(&zbars[k & 1], zpar[k & 1])) {
@@ -536,7 +538,8 @@ __global__ void __launch_bounds__(32 * WPB, 1) hmvm_tc_kernel(TcArgs ta) {
       cur_oidx = nxt_oidx;
       cur_scale = nxt_scale;
       nxt = nn;
-      nxt_seg = (has_nn && lane < nn.nseg) ? segs[nn.seg_begin + lane] : szero;
+      nxt_seg = nn_seg;
+      nn = nnn;
     }
     if (failed) {
       // let the copies and MMAs in flight finish (bounded) before the shared
