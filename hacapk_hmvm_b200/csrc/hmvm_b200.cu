@@ -670,7 +670,7 @@ int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** 
       if (e != cudaSuccess) rc = cuda_fail(e, "partial buffer");
     }
     if (!rc && L->mixed) {
-      cudaError_t e = cudaMalloc(&p->d_x32, (size_t)(L->nd + 16) * sizeof(float));
+      cudaError_t e = cudaMalloc(&p->d_x32, (size_t)x32_stride(L->nd) * 4 * sizeof(float));
       if (e != cudaSuccess) rc = cuda_fail(e, "x32 buffer");
       if (!rc) rc = upload(&p->d_scale, L->rowscale.data(), L->rowscale.size() * sizeof(double), nullptr);
     }
@@ -751,7 +751,7 @@ int launch_validate(bool& first, hmvm_plan* p, int stage, cudaStream_t st) {
 
 // Mixed plans: x rounded to FP32, V stage (scaled t in FP32), its reduction,
 // row stage, its reduction into y (partials in FP64).
-int launch_stages_mixed(hmvm_plan* p, const void* x, void* y, void* tbuf, void* pbuf, float* x32, cudaStream_t st) {
+int launch_stages_mixed(hmvm_plan* p, const void* x, void* y, void* tbuf, void* pbuf, cudaStream_t st) {
   TileArgs a;
   a.err = p->d_err;
   a.tiles = p->d_tiles;
@@ -762,7 +762,8 @@ int launch_stages_mixed(hmvm_plan* p, const void* x, void* y, void* tbuf, void* 
   a.y = y;
   a.p = pbuf;
   a.out_idx = p->d_out_idx;
-  a.x32 = x32;
+  a.x32 = p->d_x32;
+  a.x32_ld = x32_stride(p->nd);
   const int ctas = p->num_sms * p->ctas_per_sm, ctas2 = p->num_sms * p->ctas2_per_sm;
   cudaEvent_t* ev = nullptr;
   if (p->profiling && p->prof_count < kMaxProfiled) {
@@ -772,7 +773,7 @@ int launch_stages_mixed(hmvm_plan* p, const void* x, void* y, void* tbuf, void* 
   if (ev) cudaEventRecord(ev[0], st);
   bool first = true;
   HMVM_CUDA_TRY(launch_in_apply(first, hmvm_round_f32_kernel, (unsigned)std::min((p->nd + 255) / 256, p->num_sms * 8),
-                                256, 0, st, static_cast<const double*>(x), x32, p->nd),
+                                256, 0, st, static_cast<const double*>(x), p->d_x32, a.x32_ld, p->nd),
                 "x rounding launch");
   if (p->stage1_tiles > 0) {
     int vrc = launch_validate(first, p, 1, st);
@@ -826,6 +827,7 @@ int launch_stages(hmvm_plan* p, const void* x, void* y, void* tbuf, void* pbuf, 
   a.p = pbuf;
   a.out_idx = p->d_out_idx;
   a.x32 = nullptr;
+  a.x32_ld = 0;
   a.scale = nullptr;
   const int ctas = p->num_sms * p->ctas_per_sm, ctas2 = p->num_sms * p->ctas2_per_sm;
   cudaEvent_t* ev = nullptr;
@@ -1282,7 +1284,7 @@ int check_multi(const hmvm_plan* p, const void* X, int64_t ldx, const void* Y, i
 int apply_impl(hmvm_plan* p, const void* x, void* y, cudaStream_t st) {
   if (p->nd == 0) return HMVM_OK;
   if (p->tcw) return launch_tcw_pass(p, x, p->nd, y, p->nd, 1, st);  // one right-hand side in a pass
-  if (p->mixed) return launch_stages_mixed(p, x, y, p->d_t, p->d_p, p->d_x32, st);
+  if (p->mixed) return launch_stages_mixed(p, x, y, p->d_t, p->d_p, st);
   if (p->precision == HMVM_FP64) return launch_stages<double>(p, x, y, p->d_t, p->d_p, st);
   return launch_stages<float>(p, x, y, p->d_t, p->d_p, st);
 }
@@ -1811,7 +1813,7 @@ int hmvm_b200_apply_noalloc(hmvm_plan* p, const void* x, void* y, void* stream) 
   // t's padding slots must read as zero, and earlier calls (of any plan) left
   // other values there; the partial sums are written in full before they are read.
   HMVM_CUDA_TRY(cudaMemsetAsync(tbuf, 0, tbytes, st), "clear the no-alloc scratch");
-  if (p->mixed) return launch_stages_mixed(p, x, y, tbuf, pbuf, reinterpret_cast<float*>(pbuf + pbytes), st);
+  if (p->mixed) return launch_stages_mixed(p, x, y, tbuf, pbuf, st);
   if (p->precision == HMVM_FP64) return launch_stages<double>(p, x, y, tbuf, pbuf, st);
   return launch_stages<float>(p, x, y, tbuf, pbuf, st);
 }

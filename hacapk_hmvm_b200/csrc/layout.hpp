@@ -146,7 +146,11 @@ constexpr MixedCfg kMixedCfgs[kNumMixedCfgs] = {{8, 4, 2048, 2048}, {8, 4, 1024,
                                                 {4, 4, 2048, 4096}, {6, 4, 2048, 4096}, {16, 4, 1024, 2048},
                                                 {8, 2, 4096, 2048}, {4, 4, 4096, 2048}, {6, 2, 4096, 4096},
                                                 {4, 2, 8192, 2048}, {5, 2, 8192, 2048}};
-inline int mixed_smem_bytes(const MixedCfg& c) { return c.wpb * (c.slots * c.chunk + 2 * c.zbytes + c.slots * 8); }
+inline int mixed_smem_bytes(const MixedCfg& c) {
+  return c.wpb * (c.slots * c.chunk + 2 * c.zbytes + (c.slots + 2) * 8);
+}
+// Elements of each of the four copies of x rounded to FP32 (hmvm_round_f32_kernel).
+inline int64_t x32_stride(int64_t nd) { return (nd + 31) / 16 * 16; }
 // Default configuration of a stage (1: V stage, 2: row stage) for a plan's
 // precision and kernel variant.  Stream kernel: 4 warps x 16 KB rings for FP64
 // and for the FP32 V stage; the FP32 row stage runs fastest with 4 warps x
