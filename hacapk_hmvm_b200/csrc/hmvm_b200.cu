@@ -638,7 +638,7 @@ int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** 
     p->stage1_teams = lsms * p->ctas_per_sm * teams_per_cta(p->kernel, p->stage1_cfg);
     p->stage2_teams = lsms * p->ctas2_per_sm * teams_per_cta(p->kernel, p->stage2_cfg);
     std::vector<int64_t> cost;
-    for (const hmvm_tile_desc& d : L->tiles) cost.push_back((int64_t)d.nvec * d.nrows * 16 + kItemOverheadBytes);
+    for (const hmvm_tile_desc& d : L->tiles) cost.push_back((int64_t)d.nvec * 16 * (d.nrows + kItemVecRows) + kItemOverheadBytes);
     const auto mid = cost.begin() + L->stage1_tiles;
     tb1 = even_ranges(std::vector<int64_t>(cost.begin(), mid), p->stage1_teams);
     tb2 = even_ranges(std::vector<int64_t>(mid, cost.end()), p->stage2_teams);

@@ -507,7 +507,8 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
       int32_t nteams = st == 0 ? L.stage1_teams : L.stage2_teams;
       max_item[st] = stage_bytes[st] < kSmallStageBytes
                          ? std::max<int64_t>(kSmallItemBytes, stage_bytes[st] / std::max<int64_t>(1, (int64_t)nteams))
-                         : std::max<int64_t>(kMinItemBytes, stage_bytes[st] / std::max<int64_t>(1, (int64_t)nteams * kItemsPerTeam));
+                         : std::max<int64_t>(!L.mixed && stage_bytes[st] < kMidStageBytes ? kMidItemBytes : kMinItemBytes,
+                                             stage_bytes[st] / std::max<int64_t>(1, (int64_t)nteams * kItemsPerTeam));
     }
     struct Item {
       int32_t tile, va, vb, mode, out_base;
@@ -518,6 +519,9 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
     std::vector<int32_t> tile_item0(ntb + 1);
     int64_t p_len = 0;
     const bool runs = !L.mixed && nrhs_max > 1;
+    auto item_cost = [&](int32_t nvec, int32_t rows) {
+      return (int64_t)nvec * 16 * (rows + (L.mixed ? kItemVecRowsMixed : kItemVecRows)) + kItemOverheadBytes;
+    };
     for (int32_t k = 0; k < ntb; k++) {
       const TileBuild &t = tb[k];
       tile_item0[k] = (int32_t)items.size();
@@ -585,7 +589,7 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
       }
       const int32_t nparts = (int32_t)cuts.size() + 1;
       if (nparts <= 1) {
-        items.push_back(Item{k, 0, t.nvec, t.mode, t.out_base, bytes + kItemOverheadBytes});
+        items.push_back(Item{k, 0, t.nvec, t.mode, t.out_base, item_cost(t.nvec, t.nrows)});
         continue;
       }
       // part q of the tile writes its R partial sums at pb + q*R
@@ -601,7 +605,7 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
       for (int32_t q = 0; q < nparts; q++) {
         int32_t va = q == 0 ? 0 : cuts[q - 1], vb = q + 1 < nparts ? cuts[q] : t.nvec;
         items.push_back(Item{k, va, vb, 2, (int32_t)(pb + (int64_t)q * t.nrows),
-                             (int64_t)(vb - va) * t.nrows * 16 + kItemOverheadBytes});
+                             item_cost(vb - va, t.nrows)});
       }
     }
     tile_item0[ntb] = (int32_t)items.size();
@@ -627,7 +631,7 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
         std::vector<int64_t> cost(count);
         for (int32_t k = 0; k < count; k++) {
           const Item &it = items[first + k];
-          cost[k] = (int64_t)(it.vb - it.va) * 16 * (tb[it.tile].nrows + kDmmaStepRows) + kDmmaPartCost +
+          cost[k] = (int64_t)(it.vb - it.va) * 16 * (tb[it.tile].nrows + kItemVecRows) + kDmmaPartCost +
                     (it.va == 0 ? kDmmaTileCost : 0);
         }
         order = idx;

@@ -121,7 +121,20 @@ constexpr int64_t kMinItemBytes = 32 * 1024;
 constexpr int64_t kSmallStageBytes = 8 << 20;
 constexpr int64_t kSmallItemBytes = 4 * 1024;
 constexpr int64_t kItemsPerTeam = 6;
-constexpr int64_t kItemOverheadBytes = 1024;
+// Plain plans' stages below kMidStageBytes (under 28 KB per team): items down to
+// kMidItemBytes, since there a team holds one or two items of kMinItemBytes and
+// half of the teams wait.  N = 1,536 FP64, captured: 14.6 us (17.6 with 32 KiB
+// items); N = 5,000: 23.4 (24.8).  Above it the partial sums cost more: a 36 MB
+// and a 76 MB stage 31.6 against 30.5 us.  (Mixed plans keep their items: their
+// FP32 sums run per item.)
+constexpr int64_t kMidStageBytes = 32 << 20;
+constexpr int64_t kMidItemBytes = 16 * 1024;
+// An item's cost in bytes when the teams get their items: its vectors as if they
+// had kItemVecRows more rows of 16 bytes (a vector costs a warp something whatever
+// its rows; mixed kernels decode), and a fixed part.  N = 21,600 FP64, captured:
+// 54.8 us; by bytes and 1 KiB alone 59.5.  N = 131,072 mixed: 196.5 against 203.1 us.
+constexpr int kItemVecRows = 8, kItemVecRowsMixed = 16;
+constexpr int64_t kItemOverheadBytes = 4096;
 
 // Element type of a segment's matrix data (mixed-precision plans encode it in
 // the top bits of hmvm_seg_desc.ncols; plain plans leave those bits zero).
@@ -199,10 +212,9 @@ constexpr int kDmmaPageBytes = 4096;
 constexpr int kDmmaRingPad = 512;
 constexpr int kDmmaWarpsPerSm = 12;
 // Cost of an item's part in bytes when its teams get their ranges: its vectors of
-// nrows + kDmmaStepRows rows, kDmmaPartCost, and kDmmaTileCost for a tile's first
+// nrows + kItemVecRows rows, kDmmaPartCost, and kDmmaTileCost for a tile's first
 // part.  V stage of 8 FP32 right-hand sides (N = 100,003): 86 us; with 4 KiB less
 // per tile 105, with 8 KiB more 95, without the rows' share 112.
-constexpr int kDmmaStepRows = 8;
 constexpr int64_t kDmmaPartCost = 2048, kDmmaTileCost = 4096;
 constexpr int dmma_smem_bytes(const MultiCfg& c) {
   return c.wpb * (c.slots * c.chunk + kDmmaRingPad + 2 * kDmmaPageBytes + (c.slots + 2) * 8);
