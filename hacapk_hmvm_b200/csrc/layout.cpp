@@ -128,22 +128,27 @@ int validate_leaves(const LeafTable &lt, std::string &msg) {
 }
 
 std::vector<int32_t> even_ranges(const std::vector<int64_t> &cost, int n) {
-  int64_t lo = 0, hi = 0;
-  for (int64_t c : cost) {
-    lo = std::max(lo, c);
-    hi += c;
-  }
-  lo = std::max(lo, hi / std::max(n, 1));
   const int32_t count = (int32_t)cost.size();
+  std::vector<int64_t> upto((size_t)count + 1, 0);  // cost of the items before each
+  int64_t lo = 0;
+  for (int32_t i = 0; i < count; i++) {
+    upto[i + 1] = upto[i] + cost[i];
+    lo = std::max(lo, cost[i]);
+  }
+  int64_t hi = upto[count];
+  const int64_t even = hi / std::max(n, 1), close = even / 1024;
+  lo = std::max(lo, even);
   auto cut = [&](int64_t cap, std::vector<int32_t> *out) {  // ranges of at most cap
     int used = 0;
     for (int32_t i = 0; i < count; used++) {
       if (out) out->push_back(i);
-      for (int64_t c = cost[i++]; i < count && c + cost[i] <= cap; i++) c += cost[i];
+      if (used > n) return used;
+      i = (int32_t)(std::upper_bound(upto.begin() + i + 1, upto.end(), upto[i] + cap) - upto.begin()) - 1;
     }
     return used;
   };
-  while (lo < hi) {
+  hi = std::max(lo, std::min(hi, lo * 2));  // a range never needs twice the larger of the two bounds
+  while (lo + close < hi) {
     const int64_t mid = lo + (hi - lo) / 2;
     if (cut(mid, nullptr) <= n) hi = mid;
     else lo = mid + 1;

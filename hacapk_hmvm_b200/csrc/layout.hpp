@@ -315,7 +315,8 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
 int validate_leaves(const LeafTable &lt, std::string &msg);
 
 // Items of these costs, in order, cut into n ranges whose largest cost is as
-// small as whole items allow: n + 1 bounds (the last ranges may be empty).
+// small as whole items allow (to 1/1024 of the mean): n + 1 bounds (the last
+// ranges may be empty).
 std::vector<int32_t> even_ranges(const std::vector<int64_t> &cost, int n);
 
 // The wide tensor-core layout (see layout_tc.cpp).
