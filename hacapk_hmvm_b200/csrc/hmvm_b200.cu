@@ -931,14 +931,13 @@ void launch_reduce_multi(int nr_inst, const int4* red, int n, const void* pbuf, 
 
 template <int NR>
 void launch_pack(const hmvm_plan* p, const void* X, int64_t ldx, int nr, cudaStream_t st) {
-  const int64_t work = (int64_t)(p->nd + 16) * NR;
-  const int blocks = (int)std::min<int64_t>((work + 255) / 256, (int64_t)p->num_sms * 8);
+  const int blocks = (int)std::min<int64_t>(((int64_t)p->nd + 16 + kPackRows - 1) / kPackRows, (int64_t)p->num_sms * 8);
   double* x64 = p->precision != HMVM_FP32 ? p->d_xm64 : nullptr;
   float* x32 = p->precision != HMVM_FP64 ? p->d_xm32 : nullptr;
   if (p->precision == HMVM_FP32)
-    hmvm_pack_x_kernel<float, NR><<<blocks, 256, 0, st>>>(static_cast<const float*>(X), ldx, p->nd, 16, nr, x64, x32);
+    hmvm_pack_x_kernel<float, NR><<<blocks, kPackThreads, 0, st>>>(static_cast<const float*>(X), ldx, p->nd, 16, nr, x64, x32);
   else
-    hmvm_pack_x_kernel<double, NR><<<blocks, 256, 0, st>>>(static_cast<const double*>(X), ldx, p->nd, 16, nr, x64,
+    hmvm_pack_x_kernel<double, NR><<<blocks, kPackThreads, 0, st>>>(static_cast<const double*>(X), ldx, p->nd, 16, nr, x64,
                                                            x32);
 }
 
@@ -1057,13 +1056,14 @@ int tc_prepare(const hmvm_plan* p) {
 // its reduction, t into planes, row stage, its reduction into Y.
 int launch_tc_pass(hmvm_plan* p, const void* X, int64_t ldx, void* Y, int64_t ldy, int nr, cudaStream_t st) {
   const bool bf = p->mixed_kcode == 3;
-  const int gsm = p->num_sms * 8;  // grid stride (x 256 threads) is a multiple of 16, as the plane kernels need
+  const int gsm = p->num_sms * 8;  // the grid stride is a multiple of 16 bytes x 4 and of 2 halves, as these kernels need
   HMVM_CUDA_TRY(cudaMemsetAsync(p->d_amax, 0, 32 * sizeof(unsigned), st), "scale reset");
   launch_pack<kTcNrhs>(p, X, ldx, nr, st);
+  const float4* x4 = reinterpret_cast<const float4*>(p->d_xm32);
   const int64_t nx = (int64_t)(p->nd + 16) * kTcNrhs, nt = (int64_t)(p->t_len + 16) * kTcNrhs;
-  hmvm_absmax_kernel<<<gsm, 256, 0, st>>>(p->d_xm32, nx, p->d_amax);
-  if (bf) hmvm_tc_planes_kernel<true><<<gsm, 256, 0, st>>>(p->d_xm32, p->nd, 16, p->d_amax, p->d_xplanes, p->d_scal);
-  else hmvm_tc_planes_kernel<false><<<gsm, 256, 0, st>>>(p->d_xm32, p->nd, 16, p->d_amax, p->d_xplanes, p->d_scal);
+  hmvm_absmax_kernel<<<gsm, kTcAuxThreads, 0, st>>>(x4, nx, p->d_amax);
+  if (bf) hmvm_tc_planes_kernel<true><<<gsm, kTcAuxThreads, 0, st>>>(x4, p->nd, 16, p->d_amax, p->d_xplanes, p->d_scal);
+  else hmvm_tc_planes_kernel<false><<<gsm, kTcAuxThreads, 0, st>>>(x4, p->nd, 16, p->d_amax, p->d_xplanes, p->d_scal);
   HMVM_CUDA_TRY(cudaGetLastError(), "input planes launch");
   TcArgs ta;
   MultiArgs& a = ta.m;
@@ -1100,12 +1100,13 @@ int launch_tc_pass(hmvm_plan* p, const void* X, int64_t ldx, void* Y, int64_t ld
   if (ev) cudaEventRecord(ev[1], st);
   if (p->n_red1 > 0)
     launch_reduce_multi<double, float, true>(kTcNrhs, p->d_red1, p->n_red1, p->d_pm, p->d_tm, 0, nr, st);
-  hmvm_absmax_kernel<<<gsm, 256, 0, st>>>(static_cast<const float*>(p->d_tm), nt, p->d_amax + 16);
+  const float4* t4 = static_cast<const float4*>(p->d_tm);
+  hmvm_absmax_kernel<<<gsm, kTcAuxThreads, 0, st>>>(t4, nt, p->d_amax + 16);
   if (bf)
-    hmvm_tc_planes_kernel<true><<<gsm, 256, 0, st>>>(static_cast<const float*>(p->d_tm), (int)p->t_len, 16,
+    hmvm_tc_planes_kernel<true><<<gsm, kTcAuxThreads, 0, st>>>(t4, (int)p->t_len, 16,
                                                     p->d_amax + 16, p->d_tplanes, p->d_scal + 32);
   else
-    hmvm_tc_planes_kernel<false><<<gsm, 256, 0, st>>>(static_cast<const float*>(p->d_tm), (int)p->t_len, 16,
+    hmvm_tc_planes_kernel<false><<<gsm, kTcAuxThreads, 0, st>>>(t4, (int)p->t_len, 16,
                                                      p->d_amax + 16, p->d_tplanes, p->d_scal + 32);
   HMVM_CUDA_TRY(cudaGetLastError(), "t planes launch");
   if (ev) cudaEventRecord(ev[2], st);

@@ -40,15 +40,36 @@ constexpr int kTcStageBytes = kTcPiece * 32 * 16;  // 4 KiB A staging per warp
 constexpr int kTcPad = 2048;          // slack before the staging tiles (M rows below 32q)
 
 // ---- global inputs as 16-bit hi/lo planes -----------------------------------
-// amax[r] = max |v| of right-hand side r (values v[i * 16 + r]) as float bits
-// (atomicMax on the non-negative bit pattern).  The grid stride is a multiple
-// of 16, so each thread always reads the same column r = threadIdx.x % 16.
-__global__ void hmvm_absmax_kernel(const float* __restrict__ v, int64_t n, unsigned* __restrict__ amax) {
-  float m = 0.f;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    m = fmaxf(m, fabsf(v[i]));
-  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));  // lanes l and l + 16 hold the same column
-  if ((threadIdx.x & 31) < 16 && m > 0.f) atomicMax(amax + (threadIdx.x & 15), __float_as_uint(m));
+// amax[r] = max |v| of right-hand side r (values v[i * 16 + r], n a multiple of
+// 16) as float bits (atomicMax on the non-negative bit pattern).  A thread reads
+// 16 bytes at a time, always the same 4 columns; one atomic per block and column
+// (one per warp and column took 13-14 us at 4-16 MB, this 5).
+constexpr int kTcAuxThreads = 256;
+__global__ void __launch_bounds__(kTcAuxThreads) hmvm_absmax_kernel(const float4* __restrict__ v, int64_t n,
+                                                                    unsigned* __restrict__ amax) {
+  __shared__ float wm[kTcAuxThreads / 32][kTcNr];
+  float m[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n / 4; i += (int64_t)gridDim.x * blockDim.x) {
+    const float4 q = v[i];
+    m[0] = fmaxf(m[0], fabsf(q.x));
+    m[1] = fmaxf(m[1], fabsf(q.y));
+    m[2] = fmaxf(m[2], fabsf(q.z));
+    m[3] = fmaxf(m[3], fabsf(q.w));
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) m[c] = fmaxf(m[c], __shfl_xor_sync(0xffffffffu, m[c], o));
+    if (lane < 4) wm[warp][lane * 4 + c] = m[c];
+  }
+  __syncthreads();
+  if (threadIdx.x < kTcNr) {
+    float b = 0.f;
+#pragma unroll
+    for (int w = 0; w < kTcAuxThreads / 32; w++) b = fmaxf(b, wm[w][threadIdx.x]);
+    if (b > 0.f) atomicMax(amax + threadIdx.x, __float_as_uint(b));
+  }
 }
 
 // A power-of-two scale s = 2^-e with max |v| * s in [2^13, 2^14) (1 if max = 0
@@ -71,36 +92,59 @@ __device__ __forceinline__ void tc_scale(unsigned amax_bits, float* s, float* in
 // hi (g < 2) or lo (g >= 2) parts of rhs 8 * (g % 2) .. + 7, each column r
 // scaled by its own power of two s_r (from amax[r]).  Rows [n, n + pad) are
 // zero.  scal[r] = s_r, scal[16 + r] = 1 / s_r.
+// A thread takes 8 columns of a row: 32 bytes in, 16 bytes to the hi and to the
+// lo plane (2-byte stores of one value per thread took 7 and 12 us for x and t at
+// N = 65,536, this 4 and 7).
 template <bool BF>
-__global__ void hmvm_tc_planes_kernel(const float* __restrict__ src, int n, int pad, const unsigned* __restrict__ amax,
-                                      uint16_t* __restrict__ planes, float* __restrict__ scal) {
-  const int r = threadIdx.x & 15;  // the grid stride is a multiple of 16: a fixed column per thread
-  float s, inv;
-  tc_scale(amax[r], &s, &inv);
-  if (blockIdx.x == 0 && threadIdx.x < 16) {
-    scal[r] = s;
-    scal[16 + r] = inv;
-  }
-  const int64_t rows = (int64_t)n + pad;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < rows * kTcNr;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = k / kTcNr;
-    const float v = i < n ? src[k] * s : 0.f;
-    uint16_t hi, lo;
-    if (BF) {
-      const __nv_bfloat16 h = __float2bfloat16_rn(v);
-      const __nv_bfloat16 l = __float2bfloat16_rn(v - __bfloat162float(h));
-      hi = *reinterpret_cast<const uint16_t*>(&h);
-      lo = *reinterpret_cast<const uint16_t*>(&l);
-    } else {
-      const __half h = __float2half_rn(v);
-      const __half l = __float2half_rn(v - __half2float(h));
-      hi = *reinterpret_cast<const uint16_t*>(&h);
-      lo = *reinterpret_cast<const uint16_t*>(&l);
+__global__ void __launch_bounds__(kTcAuxThreads) hmvm_tc_planes_kernel(const float4* __restrict__ src, int n, int pad,
+                                                                       const unsigned* __restrict__ amax,
+                                                                       uint16_t* __restrict__ planes,
+                                                                       float* __restrict__ scal) {
+  __shared__ float scale[kTcNr];
+  if (threadIdx.x < kTcNr) {
+    float s, inv;
+    tc_scale(amax[threadIdx.x], &s, &inv);
+    scale[threadIdx.x] = s;
+    if (blockIdx.x == 0) {
+      scal[threadIdx.x] = s;
+      scal[16 + threadIdx.x] = inv;
     }
-    const int g = r >> 3, j = r & 7;
-    planes[((int64_t)g * rows + i) * 8 + j] = hi;
-    planes[((int64_t)(g + 2) * rows + i) * 8 + j] = lo;
+  }
+  __syncthreads();
+  const int g = threadIdx.x & 1;  // the grid stride is even: a fixed half of the columns per thread
+  float s[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) s[j] = scale[8 * g + j];
+  const int64_t rows = (int64_t)n + pad;
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < rows * 2; k += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = k >> 1;
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (i < n) {
+      const float4 a = src[2 * k], b = src[2 * k + 1];
+      v[0] = a.x * s[0];
+      v[1] = a.y * s[1];
+      v[2] = a.z * s[2];
+      v[3] = a.w * s[3];
+      v[4] = b.x * s[4];
+      v[5] = b.y * s[5];
+      v[6] = b.z * s[6];
+      v[7] = b.w * s[7];
+    }
+    __align__(16) uint16_t hi[8], lo[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      if (BF) {
+        const __nv_bfloat16 h = __float2bfloat16_rn(v[j]);
+        hi[j] = __bfloat16_as_ushort(h);
+        lo[j] = __bfloat16_as_ushort(__float2bfloat16_rn(v[j] - __bfloat162float(h)));
+      } else {
+        const __half h = __float2half_rn(v[j]);
+        hi[j] = __half_as_ushort(h);
+        lo[j] = __half_as_ushort(__float2half_rn(v[j] - __half2float(h)));
+      }
+    }
+    reinterpret_cast<uint4*>(planes)[(int64_t)g * rows + i] = *reinterpret_cast<const uint4*>(hi);
+    reinterpret_cast<uint4*>(planes)[(int64_t)(g + 2) * rows + i] = *reinterpret_cast<const uint4*>(lo);
   }
 }
 
@@ -512,23 +556,17 @@ __global__ void __launch_bounds__(32 * WPB, 1) hmvm_tc_kernel(TcArgs ta) {
       if (failed) break;
       if (lane < R) {
         if constexpr (VST) {
-          if (cur.mode == 1) {
 #pragma unroll
-            for (int r = 0; r < NR; r++)
-              static_cast<float*>(a.t)[(int64_t)cur_oidx * NR + r] = (float)(row[r] * cur_scale);
-          } else {
-#pragma unroll
-            for (int r = 0; r < NR; r++)
-              static_cast<double*>(a.p)[(int64_t)(cur.out_base + lane) * NR + r] = row[r] * cur_scale;
-          }
+          for (int r = 0; r < NR; r++) row[r] *= cur_scale;
+          if (cur.mode == 1) store_values<NR>(static_cast<float*>(a.t) + (int64_t)cur_oidx * NR, row);
+          else store_values<NR>(static_cast<double*>(a.p) + (int64_t)(cur.out_base + lane) * NR, row);
         } else {
           if (cur.mode == 0) {
 #pragma unroll
             for (int r = 0; r < NR; r++)
               if (r < a.nr) static_cast<double*>(a.y)[cur.out_base + lane + r * a.ldy] = row[r];
           } else {
-#pragma unroll
-            for (int r = 0; r < NR; r++) static_cast<double*>(a.p)[(int64_t)(cur.out_base + lane) * NR + r] = row[r];
+            store_values<NR>(static_cast<double*>(a.p) + (int64_t)(cur.out_base + lane) * NR, row);
           }
         }
       }
