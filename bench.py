@@ -372,7 +372,9 @@ def kernel_name(plan, info, nrhs):
     if info["kernel"] == 4:
         return "hmvm_tcw_kernel"
     if nrhs > 1:
-        return "hmvm_tc_kernel" if (plan.precision == "mixed" and info["nrhs_max"] >= 16) else "hmvm_multi_kernel"
+        if plan.precision != "mixed":
+            return "hmvm_dmma_kernel"
+        return "hmvm_tc_kernel" if info["nrhs_max"] >= 16 else "hmvm_multi_kernel"
     return {0: "hmvm_tile_kernel", 1: "hmvm_stream_kernel", 2: "hmvm_mixed_kernel"}[info["kernel"]]
 
 

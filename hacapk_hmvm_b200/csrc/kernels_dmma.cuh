@@ -25,17 +25,19 @@
 //
 // FP32 plans: the matrix values come from ldmatrix in the operand's layout and
 // are widened to FP64 in registers, as are the inputs, so products and sums are
-// FP64 (error against FP64 2e-7 -> 4e-8).  4 matrix and 1 conversion instruction
-// per vector more than FP64's half vector: the FP64 pipe is busy for half of the
-// row stage.  tf32 or 16-bit splits on the tensor cores would have been less
-// exact than the FP32 sums they replaced.
+// FP64 (error against FP64 2e-7 -> 4e-8).  A vector is a whole step there, so the
+// FP64 pipe is busy for half of the row stage.  tf32 or 16-bit splits on the
+// tensor cores would have been less exact than the FP32 sums they replaced.
 //
 // A team adds up the consecutive parts of a tile that it has (one page of inputs
 // each), so only tiles that two teams share have partial sums.
 //
 // Measured, 8 right-hand sides, whole apply (V stage, row stage): N = 65,536 FP64
-// sphere, 1.04 GB: 464 us (147, 295) -> 229 (77, 128: 5.3 TB/s); N = 100,003 FP32
-// cube, 0.95 GB: 401 us (133, 237) -> 256 (86, 155).
+// sphere, 1.04 GB: 464 us (147, 295) -> 227 (75, 123: 5.5 TB/s); N = 100,003 FP32
+// cube, 0.95 GB: 402 us (134, 237) -> 253 (84, 155: 3.9 TB/s).  m16n8k8 in place of
+// four m8n8k4 changed nothing (251.3 to 250.6 us), nor did leaving out the
+// conversions to FP64 (246): 12 warps waiting for dependent instructions (2.9 of 7
+// cycles each) and for their ring are what is left.
 #pragma once
 
 #include "kernels_multi.cuh"
