@@ -512,8 +512,7 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
       int32_t nteams = st == 0 ? L.stage1_teams : L.stage2_teams;
       max_item[st] = stage_bytes[st] < kSmallStageBytes
                          ? std::max<int64_t>(kSmallItemBytes, stage_bytes[st] / std::max<int64_t>(1, (int64_t)nteams))
-                         : std::max<int64_t>(!L.mixed && stage_bytes[st] < kMidStageBytes ? kMidItemBytes : kMinItemBytes,
-                                             stage_bytes[st] / std::max<int64_t>(1, (int64_t)nteams * kItemsPerTeam));
+                         : std::max<int64_t>(kMinItemBytes, stage_bytes[st] / std::max<int64_t>(1, (int64_t)nteams * kItemsPerTeam));
     }
     struct Item {
       int32_t tile, va, vb, mode, out_base;

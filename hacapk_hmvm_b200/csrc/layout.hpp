@@ -121,14 +121,6 @@ constexpr int64_t kMinItemBytes = 32 * 1024;
 constexpr int64_t kSmallStageBytes = 8 << 20;
 constexpr int64_t kSmallItemBytes = 4 * 1024;
 constexpr int64_t kItemsPerTeam = 6;
-// Plain plans' stages below kMidStageBytes (under 28 KB per team): items down to
-// kMidItemBytes, since there a team holds one or two items of kMinItemBytes and
-// half of the teams wait.  N = 1,536 FP64, captured: 14.6 us (17.6 with 32 KiB
-// items); N = 5,000: 23.4 (24.8).  Above it the partial sums cost more: a 36 MB
-// and a 76 MB stage 31.6 against 30.5 us.  (Mixed plans keep their items: their
-// FP32 sums run per item.)
-constexpr int64_t kMidStageBytes = 32 << 20;
-constexpr int64_t kMidItemBytes = 16 * 1024;
 // An item's cost in bytes when the teams get their items: its vectors as if they
 // had kItemVecRows more rows of 16 bytes (a vector costs a warp something whatever
 // its rows; mixed kernels decode), and a fixed part.  N = 21,600 FP64, captured:
