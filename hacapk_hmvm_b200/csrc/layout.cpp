@@ -642,7 +642,12 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
         team_begin = even_ranges(cost, nteams);
         return;
       }
-      std::stable_sort(idx.begin(), idx.end(), [&](int32_t a, int32_t b) { return items[a].cost > items[b].cost; });
+      // largest first; by bytes alone where no team gets a second item
+      auto key = [&](int32_t k) {
+        const Item &it = items[k];
+        return count <= nteams ? (int64_t)(it.vb - it.va) * tb[it.tile].nrows : it.cost;
+      };
+      std::stable_sort(idx.begin(), idx.end(), [&](int32_t a, int32_t b) { return key(a) > key(b); });
       using HE = std::pair<int64_t, int32_t>;
       std::priority_queue<HE, std::vector<HE>, std::greater<HE>> heap;
       for (int32_t k = 0; k < nteams; k++) heap.emplace(0, k);
