@@ -197,7 +197,8 @@ struct hmvm_plan {
   // mixed precision
   bool mixed = false;
   int mixed_kcode = 2;  // stage_launch code: 2 FP16 factors, 3 BF16 factors
-  float* d_x32 = nullptr;
+  float* d_x32 = nullptr;    // mixed plans: x rounded to FP32, four copies
+  float* d_x32na = nullptr;  // ... those of hmvm_b200_apply_noalloc, which may overlap an apply
   double* d_scale = nullptr;
   int64_t cols_fp32 = 0, cols_lr16 = 0, cols_fp8 = 0, stored_bytes = 0;
   int t_elem = 8, p_elem = 8;  // bytes per t slot and per partial sum
@@ -281,7 +282,7 @@ void free_plan_buffers(hmvm_plan* p) {
   p->cs_in = p->cs_out = nullptr;
   p->prof_events.clear();
   void* bufs[] = {p->d_data, p->d_tiles, p->d_segs, p->d_tb1, p->d_tb2,  p->d_out_idx, p->d_red1,
-                  p->d_red2, p->d_t,     p->d_p,    p->d_err, p->d_x,    p->d_y,       p->d_x32,
+                  p->d_red2, p->d_t,     p->d_p,    p->d_err, p->d_x,    p->d_y,       p->d_x32, p->d_x32na,
                   p->d_scale, p->d_xm64, p->d_xm32, p->d_tm,  p->d_pm,   p->d_xh,      p->d_yh,
                   p->d_xplanes, p->d_tplanes, p->d_scal, p->d_amax, p->d_xpl, p->d_tpl,
                   p->d_tscale, p->d_xscale, p->d_amax128, p->d_part, p->d_tblocks, p->d_tgroups,
@@ -438,8 +439,6 @@ int tcw_buffers(hmvm_plan* p, const HostLayout& L) {
   return rc;
 }
 
-// sms_cap > 0: plan the layout's teams for that many SMs (a batch class shares the GPU
-// with the other classes of its batch, which run in the same launches).
 // The input buffer of a stage's kernel for a layout's shapes, in bytes, as the
 // planner bounds items by it (0: the kernel has none, or the layout is the
 // wide tensor-core one, whose items these checks do not describe).
@@ -521,6 +520,21 @@ int validate_layout(const HostLayout& L, std::string& msg) {
   return HMVM_OK;
 }
 
+// What hmvm_b200_apply_noalloc counts against its scratch array: t, then the partial sums.
+struct NoallocNeed {
+  size_t t, p, total;
+};
+NoallocNeed noalloc_need(const hmvm_plan* p) {
+  auto round256 = [](size_t b) { return (b + 255) / 256 * 256; };
+  NoallocNeed n;
+  n.t = round256((size_t)(p->t_len + 16) * p->t_elem);
+  n.p = round256((size_t)(p->p_len + 16) * p->p_elem);
+  n.total = n.t + n.p + (p->mixed ? round256((size_t)(p->nd + 16) * sizeof(float)) : 0);
+  return n;
+}
+
+// sms_cap > 0: plan the layout's teams for that many SMs (a batch class shares the GPU
+// with the other classes of its batch, which run in the same launches).
 int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** out, int sms_cap = 0) {
   if (!out) return set_error(HMVM_EINVAL, "plan output pointer is NULL");
   *out = nullptr;
@@ -670,7 +684,11 @@ int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** 
       if (e != cudaSuccess) rc = cuda_fail(e, "partial buffer");
     }
     if (!rc && L->mixed) {
-      cudaError_t e = cudaMalloc(&p->d_x32, (size_t)x32_stride(L->nd) * 4 * sizeof(float));
+      const size_t xbytes = (size_t)x32_stride(L->nd) * 4 * sizeof(float);
+      cudaError_t e = cudaSuccess;
+      if (!p->tcw) e = cudaMalloc(&p->d_x32, xbytes);
+      if (e == cudaSuccess && !p->tcw && noalloc_need(p).total <= (size_t)HMVM_NOALLOC_SCRATCH_BYTES)
+        e = cudaMalloc(&p->d_x32na, xbytes);
       if (e != cudaSuccess) rc = cuda_fail(e, "x32 buffer");
       if (!rc) rc = upload(&p->d_scale, L->rowscale.data(), L->rowscale.size() * sizeof(double), nullptr);
     }
@@ -751,7 +769,7 @@ int launch_validate(bool& first, hmvm_plan* p, int stage, cudaStream_t st) {
 
 // Mixed plans: x rounded to FP32, V stage (scaled t in FP32), its reduction,
 // row stage, its reduction into y (partials in FP64).
-int launch_stages_mixed(hmvm_plan* p, const void* x, void* y, void* tbuf, void* pbuf, cudaStream_t st) {
+int launch_stages_mixed(hmvm_plan* p, const void* x, void* y, void* tbuf, void* pbuf, float* x32, cudaStream_t st) {
   TileArgs a;
   a.err = p->d_err;
   a.tiles = p->d_tiles;
@@ -762,7 +780,7 @@ int launch_stages_mixed(hmvm_plan* p, const void* x, void* y, void* tbuf, void* 
   a.y = y;
   a.p = pbuf;
   a.out_idx = p->d_out_idx;
-  a.x32 = p->d_x32;
+  a.x32 = x32;
   a.x32_ld = x32_stride(p->nd);
   const int ctas = p->num_sms * p->ctas_per_sm, ctas2 = p->num_sms * p->ctas2_per_sm;
   cudaEvent_t* ev = nullptr;
@@ -773,7 +791,7 @@ int launch_stages_mixed(hmvm_plan* p, const void* x, void* y, void* tbuf, void* 
   if (ev) cudaEventRecord(ev[0], st);
   bool first = true;
   HMVM_CUDA_TRY(launch_in_apply(first, hmvm_round_f32_kernel, (unsigned)std::min((p->nd + 255) / 256, p->num_sms * 8),
-                                256, 0, st, static_cast<const double*>(x), p->d_x32, a.x32_ld, p->nd),
+                                256, 0, st, static_cast<const double*>(x), x32, a.x32_ld, p->nd),
                 "x rounding launch");
   if (p->stage1_tiles > 0) {
     int vrc = launch_validate(first, p, 1, st);
@@ -1285,7 +1303,7 @@ int check_multi(const hmvm_plan* p, const void* X, int64_t ldx, const void* Y, i
 int apply_impl(hmvm_plan* p, const void* x, void* y, cudaStream_t st) {
   if (p->nd == 0) return HMVM_OK;
   if (p->tcw) return launch_tcw_pass(p, x, p->nd, y, p->nd, 1, st);  // one right-hand side in a pass
-  if (p->mixed) return launch_stages_mixed(p, x, y, p->d_t, p->d_p, st);
+  if (p->mixed) return launch_stages_mixed(p, x, y, p->d_t, p->d_p, p->d_x32, st);
   if (p->precision == HMVM_FP64) return launch_stages<double>(p, x, y, p->d_t, p->d_p, st);
   return launch_stages<float>(p, x, y, p->d_t, p->d_p, st);
 }
@@ -1793,12 +1811,9 @@ int hmvm_b200_apply_noalloc(hmvm_plan* p, const void* x, void* y, void* stream) 
   int rc = check_xy(p, x, y);
   if (rc) return rc;
   if (p->tcw) return set_error(HMVM_EINVAL, "tensor-core multi-RHS plans keep their scratch in the plan; use hmvm_b200_apply");
-  auto round256 = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t tbytes = round256((size_t)(p->t_len + 16) * p->t_elem);
-  const size_t pbytes = round256((size_t)(p->p_len + 16) * p->p_elem);
-  const size_t xbytes = p->mixed ? round256((size_t)(p->nd + 16) * sizeof(float)) : 0;
-  if (tbytes + pbytes + xbytes > (size_t)HMVM_NOALLOC_SCRATCH_BYTES)
-    return set_error(HMVM_ERANGE, "this plan needs " + std::to_string(tbytes + pbytes + xbytes) +
+  const NoallocNeed need = noalloc_need(p);
+  if (need.total > (size_t)HMVM_NOALLOC_SCRATCH_BYTES)
+    return set_error(HMVM_ERANGE, "this plan needs " + std::to_string(need.total) +
                                       " bytes of scratch but hmvm_b200_apply_noalloc has " +
                                       std::to_string((size_t)HMVM_NOALLOC_SCRATCH_BYTES) +
                                       "; use hmvm_b200_apply");
@@ -1809,12 +1824,12 @@ int hmvm_b200_apply_noalloc(hmvm_plan* p, const void* x, void* y, void* stream) 
   rc = noalloc_scratch(p->device, &base);
   if (rc) return rc;
   char* tbuf = static_cast<char*>(base);
-  char* pbuf = tbuf + tbytes;
+  char* pbuf = tbuf + need.t;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // t's padding slots must read as zero, and earlier calls (of any plan) left
   // other values there; the partial sums are written in full before they are read.
-  HMVM_CUDA_TRY(cudaMemsetAsync(tbuf, 0, tbytes, st), "clear the no-alloc scratch");
-  if (p->mixed) return launch_stages_mixed(p, x, y, tbuf, pbuf, st);
+  HMVM_CUDA_TRY(cudaMemsetAsync(tbuf, 0, need.t, st), "clear the no-alloc scratch");
+  if (p->mixed) return launch_stages_mixed(p, x, y, tbuf, pbuf, p->d_x32na, st);
   if (p->precision == HMVM_FP64) return launch_stages<double>(p, x, y, tbuf, pbuf, st);
   return launch_stages<float>(p, x, y, tbuf, pbuf, st);
 }

@@ -385,7 +385,10 @@ int hmvm_b200_autotune_cached64(const hmvm_leaves64 *lv, int32_t rowmat_is_float
  * `stream` and before its kernels, the part that has to start at zero.  Calls
  * whose work overlaps on the GPU (other streams, threads or plans running at
  * the same time) race on the array; order them on one stream or synchronise
- * between them.  No counterpart in the reference. */
+ * between them.  A mixed plan's rounded copies of x for this call lie in the
+ * plan (16 bytes per unknown, allocated with it) apart from hmvm_b200_apply's,
+ * so an hmvm_b200_apply or replay of the same plan may overlap this call.  No
+ * counterpart in the reference. */
 int hmvm_b200_apply_noalloc(hmvm_plan *plan, const void *x_dev, void *y_dev, void *stream);
 
 /* Per-stage device timing.  While enabled, every apply records CUDA events
