@@ -529,7 +529,7 @@ NoallocNeed noalloc_need(const hmvm_plan* p) {
   NoallocNeed n;
   n.t = round256((size_t)(p->t_len + 16) * p->t_elem);
   n.p = round256((size_t)(p->p_len + 16) * p->p_elem);
-  n.total = n.t + n.p + (p->mixed ? round256((size_t)(p->nd + 16) * sizeof(float)) : 0);
+  n.total = n.t + n.p;
   return n;
 }
 
