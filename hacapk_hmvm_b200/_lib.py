@@ -154,6 +154,15 @@ class LayoutView(C.Structure):
                 ("n_tops", C.c_int64)]
 
 
+class LayoutMultiView(C.Structure):
+    _fields_ = [("n_tiles", C.c_int32), ("n_segs", C.c_int32), ("stage1_tiles", C.c_int32),
+                ("stage1_teams", C.c_int32), ("stage2_teams", C.c_int32), ("n_red1", C.c_int32),
+                ("n_red2", C.c_int32), ("_pad0", C.c_int32),
+                ("tiles", C.c_void_p), ("segs", C.c_void_p), ("seg_first", C.POINTER(C.c_int32)),
+                ("team_begin1", C.POINTER(C.c_int32)), ("team_begin2", C.POINTER(C.c_int32)),
+                ("red1", C.POINTER(C.c_int32)), ("red2", C.POINTER(C.c_int32))]
+
+
 class HgenParams(C.Structure):
     _fields_ = [("n", C.c_int64), ("geometry", C.c_int32), ("leaf_size", C.c_int32), ("eta", C.c_double),
                 ("eps", C.c_double), ("aca_eps_factor", C.c_double), ("kmax", C.c_int32),
@@ -212,6 +221,7 @@ HMVM_SIGNATURES = {
     "hmvm_b200_layout_build64": (C.c_int, [C.POINTER(Leaves64), C.c_int32, C.POINTER(PlanOpts), C.c_int32,
                                            C.POINTER(C.c_void_p)]),
     "hmvm_b200_layout_view": (C.c_int, [C.c_void_p, C.POINTER(LayoutView)]),
+    "hmvm_b200_layout_multi_view": (C.c_int, [C.c_void_p, C.POINTER(LayoutMultiView)]),
     "hmvm_b200_layout_validate": (C.c_int, [C.c_void_p]),
     "hmvm_b200_plan_descriptors": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p), C.POINTER(C.c_int32),
                                              C.POINTER(C.c_int32)]),

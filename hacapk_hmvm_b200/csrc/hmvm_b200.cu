@@ -487,37 +487,90 @@ const char* check_name(int rc) {
   }
 }
 
-// Every descriptor of a single-vector layout against the buffers it indexes
-// (validate.hpp); wide tensor-core layouts are not described by these checks.
+// Every descriptor of a layout against the buffers it indexes (validate.hpp): the
+// items of the single-vector and mixed kernels, and those of hmvm_dmma_kernel.
+// Wide tensor-core layouts are not described by these checks.
+// One set of items and what its kernels read beside them.
+struct ItemSet {
+  const char* name;
+  const std::vector<hmvm_tile_desc>& tiles;
+  const std::vector<hmvm_seg_desc>& segs;
+  int32_t stage1_tiles, teams[2];
+  const std::vector<int32_t>*red[2], *team_begin[2];
+  int64_t zcap[2];
+  const std::vector<int32_t>* seg_first;  // hmvm_dmma_kernel's items (else NULL)
+};
+
+int validate_items(const HostLayout& L, const ItemSet& s, std::string& msg) {
+  LayoutCaps c = caps_of(L);
+  c.n_segs = (int64_t)s.segs.size();
+  c.n_tiles = (int32_t)s.tiles.size();
+  auto fail = [&](const std::string& what) {
+    msg = s.name + what;
+    return HMVM_ERANGE;
+  };
+  int64_t off = 0;  // the items cover the data stream in order
+  for (int32_t k = 0; k < (int32_t)s.tiles.size(); k++) {
+    const hmvm_tile_desc& d = s.tiles[k];
+    const int st = k < s.stage1_tiles ? 0 : 1;
+    auto bad = [&](const char* what) {
+      return fail("item " + std::to_string(k) + " (stage " + std::to_string(st + 1) + "): " + what);
+    };
+    const int rc = check_tile(d, s.segs.data(), L.out_idx.data(), c, L.vec, L.elem_size, s.zcap[st], st == 0);
+    if (rc) return bad(check_name(rc));
+    if (d.data_off != off) return bad("its data does not follow the item before it");
+    off += (int64_t)d.nvec * d.nrows;
+    int32_t col = 0;
+    for (int32_t j = d.seg_begin; s.seg_first && j < d.seg_begin + d.nseg; j++) {
+      if ((*s.seg_first)[j] != col) return bad("a segment does not start at its first column");
+      col += (s.segs[j].ncols + L.vec - 1) / L.vec * L.vec;
+    }
+  }
+  if (off != (int64_t)L.data.size()) return fail("the items do not cover the data stream");
+  // Every output once: written by an item, or added up from partial sums, each of
+  // which one item writes and one reduction entry reads.
+  std::vector<uint8_t> part((size_t)L.p_len, 0);
+  for (int st = 0; st < 2; st++) {
+    const std::string stage = "stage " + std::to_string(st + 1);
+    std::vector<uint8_t> out((size_t)(st == 0 ? L.t_len : (int64_t)L.nd), 0);
+    const int32_t first = st == 0 ? 0 : s.stage1_tiles, end = st == 0 ? s.stage1_tiles : c.n_tiles;
+    for (int32_t k = first; k < end; k++)
+      for (int32_t r = s.tiles[k].out_base; r < s.tiles[k].out_base + s.tiles[k].nrows; r++) {
+        uint8_t& w = s.tiles[k].mode == 2 ? part[r] : out[s.tiles[k].mode == 1 ? L.out_idx[r] : r];
+        if (w++) return fail("item " + std::to_string(k) + " (" + stage + "): another item writes its outputs");
+      }
+    const std::vector<int32_t>& red = *s.red[st];
+    for (size_t e = 0; e + 4 <= red.size(); e += 4) {
+      auto bad = [&](const char* what) { return fail("reduction entry " + std::to_string(e / 4) + " of " + stage + what); };
+      if (check_red(&red[e], c, st == 0)) return bad(" reads or writes outside its buffers");
+      for (int32_t q = 0; q < red[e + 2]; q++)
+        if (part[red[e + 1] + q * red[e + 3]]++ != 1) return bad(" reads a partial sum that is not its own");
+      if (out[red[e]]++) return bad(" writes an output that is written already");
+    }
+    if (st == 1 && std::count(out.begin(), out.end(), 1) != (int64_t)out.size())
+      return fail("a row of y is not written");
+    const std::vector<int32_t>& tb = *s.team_begin[st];
+    if ((int64_t)tb.size() != (int64_t)s.teams[st] + 1 || check_teams(tb.data(), s.teams[st], first, end))
+      return fail("the team ranges of " + stage + " do not cover its items in order");
+  }
+  if (std::count(part.begin(), part.end(), 1) != 0) return fail("a partial sum is written but not read");
+  return HMVM_OK;
+}
+
 int validate_layout(const HostLayout& L, std::string& msg) {
   if (L.tcw) return HMVM_OK;
-  const LayoutCaps c = caps_of(L);
-  const int64_t z1 = stage_zcap_bytes(L, 1), z2 = stage_zcap_bytes(L, 2);
-  for (int32_t k = 0; k < (int32_t)L.tiles.size(); k++) {
-    const bool st1 = k < L.stage1_tiles;
-    const int rc = check_tile(L.tiles[k], L.segs.data(), L.out_idx.data(), c, L.vec, L.elem_size, st1 ? z1 : z2, st1);
-    if (rc) {
-      msg = "item " + std::to_string(k) + " (stage " + (st1 ? "1" : "2") + "): " + check_name(rc);
-      return HMVM_ERANGE;
-    }
+  const ItemSet single = {"", L.tiles, L.segs, L.stage1_tiles, {L.stage1_teams, L.stage2_teams}, {&L.red1, &L.red2},
+                          {&L.team_begin1, &L.team_begin2}, {stage_zcap_bytes(L, 1), stage_zcap_bytes(L, 2)}, nullptr};
+  const int rc = validate_items(L, single, msg);
+  if (rc || L.mteam_begin1.empty()) return rc;
+  if (L.mseg_first.size() != L.msegs.size()) {
+    msg = "multi-RHS segments without a first column";
+    return HMVM_ERANGE;
   }
-  for (int st = 1; st <= 2; st++) {
-    const std::vector<int32_t>& red = st == 1 ? L.red1 : L.red2;
-    for (size_t e = 0; e + 4 <= red.size(); e += 4)
-      if (check_red(&red[e], c, st == 1)) {
-        msg = "reduction entry " + std::to_string(e / 4) + " of stage " + std::to_string(st) +
-              " reads or writes outside its buffers";
-        return HMVM_ERANGE;
-      }
-    const std::vector<int32_t>& tb = st == 1 ? L.team_begin1 : L.team_begin2;
-    const int32_t nt = st == 1 ? L.stage1_teams : L.stage2_teams;
-    const int32_t first = st == 1 ? 0 : L.stage1_tiles, end = st == 1 ? L.stage1_tiles : (int32_t)L.tiles.size();
-    if ((int64_t)tb.size() != (int64_t)nt + 1 || check_teams(tb.data(), nt, first, end)) {
-      msg = "the team ranges of stage " + std::to_string(st) + " do not cover its items in order";
-      return HMVM_ERANGE;
-    }
-  }
-  return HMVM_OK;
+  const ItemSet multi = {"multi-RHS ", L.mtiles, L.msegs, L.mteam_begin1.back(),
+                         {(int32_t)L.mteam_begin1.size() - 1, (int32_t)L.mteam_begin2.size() - 1},
+                         {&L.mred1, &L.mred2}, {&L.mteam_begin1, &L.mteam_begin2}, {0, 0}, &L.mseg_first};
+  return validate_items(L, multi, msg);
 }
 
 // What hmvm_b200_apply_noalloc counts against its scratch array: t, then the partial sums.
@@ -640,23 +693,12 @@ int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** 
     p->stage1_bytes = (v_elems + (int64_t)lt.nd) * L->elem_size;
     p->stage2_bytes = (L->stored_elems - v_elems + 2 * (int64_t)lt.nd) * L->elem_size;
   }
-  // A plain multi-RHS plan's teams are hmvm_dmma_kernel's; the single-vector
-  // kernels take the same items in as many ranges as they have resident teams.
   const bool plain_multi = !L->mtiles.empty();
-  std::vector<int32_t> tb1 = L->team_begin1, tb2 = L->team_begin2;
   if (plain_multi) {
-    p->mteams1 = L->stage1_teams;
-    p->mteams2 = L->stage2_teams;
+    p->mteams1 = (int32_t)L->mteam_begin1.size() - 1;
+    p->mteams2 = (int32_t)L->mteam_begin2.size() - 1;
     p->n_mred1 = (int32_t)(L->mred1.size() / 4);
     p->n_mred2 = (int32_t)(L->mred2.size() / 4);
-    p->stage1_teams = lsms * p->ctas_per_sm * teams_per_cta(p->kernel, p->stage1_cfg);
-    p->stage2_teams = lsms * p->ctas2_per_sm * teams_per_cta(p->kernel, p->stage2_cfg);
-    std::vector<int64_t> cost;
-    for (const hmvm_tile_desc& d : L->tiles) cost.push_back((int64_t)d.nvec * 16 * (d.nrows + kItemVecRows) + kItemOverheadBytes);
-    const auto mid = cost.begin() + L->stage1_tiles;
-    tb1 = even_ranges(std::vector<int64_t>(cost.begin(), mid), p->stage1_teams);
-    tb2 = even_ranges(std::vector<int64_t>(mid, cost.end()), p->stage2_teams);
-    for (int32_t& b : tb2) b += L->stage1_tiles;
   }
   {
     DeviceGuard g(dev);
@@ -666,8 +708,8 @@ int create_plan(const LeafTable& lt, const hmvm_plan_opts* opts_in, hmvm_plan** 
     p->device_bytes = dbytes;
     if (!rc) rc = upload(&p->d_tiles, L->tiles.data(), L->tiles.size() * sizeof(hmvm_tile_desc), nullptr);
     if (!rc) rc = upload(&p->d_segs, L->segs.data(), L->segs.size() * sizeof(hmvm_seg_desc), nullptr);
-    if (!rc) rc = upload(&p->d_tb1, tb1.data(), tb1.size() * 4, nullptr);
-    if (!rc) rc = upload(&p->d_tb2, tb2.data(), tb2.size() * 4, nullptr);
+    if (!rc) rc = upload(&p->d_tb1, L->team_begin1.data(), L->team_begin1.size() * 4, nullptr);
+    if (!rc) rc = upload(&p->d_tb2, L->team_begin2.data(), L->team_begin2.size() * 4, nullptr);
     if (!rc) rc = upload(&p->d_out_idx, L->out_idx.data(), L->out_idx.size() * 4, nullptr);
     if (!rc) rc = upload(&p->d_red1, L->red1.data(), L->red1.size() * 4, nullptr);
     if (!rc) rc = upload(&p->d_red2, L->red2.data(), L->red2.size() * 4, nullptr);
@@ -1891,6 +1933,28 @@ int hmvm_b200_layout_validate(const hmvm_layout* h) {
   std::string msg;
   const int rc = validate_layout(h->L, msg);
   return rc ? set_error(rc, "layout check: " + msg) : HMVM_OK;
+}
+
+int hmvm_b200_layout_multi_view(const hmvm_layout* h, hmvm_layout_multi_view* v) {
+  if (!h || !v) return set_error(HMVM_EINVAL, "NULL argument");
+  const HostLayout& L = h->L;
+  std::memset(v, 0, sizeof(*v));
+  if (L.mteam_begin1.empty()) return HMVM_OK;
+  v->n_tiles = (int32_t)L.mtiles.size();
+  v->n_segs = (int32_t)L.msegs.size();
+  v->stage1_tiles = L.mteam_begin1.back();
+  v->stage1_teams = (int32_t)L.mteam_begin1.size() - 1;
+  v->stage2_teams = (int32_t)L.mteam_begin2.size() - 1;
+  v->n_red1 = (int32_t)(L.mred1.size() / 4);
+  v->n_red2 = (int32_t)(L.mred2.size() / 4);
+  v->tiles = L.mtiles.data();
+  v->segs = L.msegs.data();
+  v->seg_first = L.mseg_first.data();
+  v->team_begin1 = L.mteam_begin1.data();
+  v->team_begin2 = L.mteam_begin2.data();
+  v->red1 = L.mred1.data();
+  v->red2 = L.mred2.data();
+  return HMVM_OK;
 }
 
 int hmvm_b200_layout_view(const hmvm_layout* h, hmvm_layout_view* v) {

@@ -498,18 +498,23 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
                      (L.mixed ? kMixedCfgs[L.stage1_cfg].wpb : teams_per_cta(L.kernel, L.stage1_cfg));
     L.stage2_teams = L.num_sms * L.ctas2_per_sm *
                      (L.mixed ? kMixedCfgs[L.stage2_cfg].wpb : teams_per_cta(L.kernel, L.stage2_cfg));
-    if (nrhs_max > 1) {
-      // teams for the multi-RHS kernel, all resident at once (mixed plans: no more than
-      // the single-vector kernels launch; plain plans give those their own ranges)
+    const bool runs = !L.mixed && nrhs_max > 1;
+    int32_t plan_teams[2] = {L.stage1_teams, L.stage2_teams};  // the teams that the items are cut for
+    if (runs) {
+      // hmvm_dmma_kernel's, all resident at once; the single-vector kernels take
+      // the same items in ranges of their own
+      plan_teams[0] = plan_teams[1] = L.num_sms * kDmmaWarpsPerSm;
+    } else if (nrhs_max > 1) {
+      // one assignment for both kernels: no more teams than either keeps resident
       const int per_sm = nrhs_max == kTcNrhs ? kTcWarpsPerSm : kMultiWarpsPerSm;
-      L.stage1_teams = L.mixed ? std::min(L.stage1_teams, L.num_sms * per_sm) : L.num_sms * kDmmaWarpsPerSm;
-      L.stage2_teams = L.mixed ? std::min(L.stage2_teams, L.num_sms * per_sm) : L.num_sms * kDmmaWarpsPerSm;
+      L.stage1_teams = plan_teams[0] = std::min(L.stage1_teams, L.num_sms * per_sm);
+      L.stage2_teams = plan_teams[1] = std::min(L.stage2_teams, L.num_sms * per_sm);
     }
     int64_t stage_bytes[2] = {0, 0};
     for (int32_t k = 0; k < ntb; k++) stage_bytes[k < n1 ? 0 : 1] += (int64_t)tb[k].nvec * tb[k].nrows * 16;
     int64_t max_item[2];
     for (int st = 0; st < 2; st++) {
-      int32_t nteams = st == 0 ? L.stage1_teams : L.stage2_teams;
+      const int32_t nteams = plan_teams[st];
       max_item[st] = stage_bytes[st] < kSmallStageBytes
                          ? std::max<int64_t>(kSmallItemBytes, stage_bytes[st] / std::max<int64_t>(1, (int64_t)nteams))
                          : std::max<int64_t>(kMinItemBytes, stage_bytes[st] / std::max<int64_t>(1, (int64_t)nteams * kItemsPerTeam));
@@ -522,7 +527,6 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
     items.reserve((size_t)ntb + ntb / 2);
     std::vector<int32_t> tile_item0(ntb + 1);
     int64_t p_len = 0;
-    const bool runs = !L.mixed && nrhs_max > 1;
     auto item_cost = [&](int32_t nvec, int32_t rows) {
       return (int64_t)nvec * 16 * (rows + (L.mixed ? kItemVecRowsMixed : kItemVecRows)) + kItemOverheadBytes;
     };
@@ -624,22 +628,24 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
 
     // ---- team assignment (LPT) and ordering --------------------------------
     auto assign = [&](int32_t first, int32_t count, int32_t nteams, std::vector<int32_t> &order,
-                      std::vector<int32_t> &team_begin) {
+                      std::vector<int32_t> &team_begin, std::vector<int32_t> &run_begin) {
       std::vector<int32_t> idx(count);
       for (int32_t k = 0; k < count; k++) idx[k] = first + k;
       if (runs) {
         // Plain multi-RHS plans: the items stay in order and are cut into ranges
-        // of about the same cost, so that a team adds up the parts of a tile that
-        // it gets.  A vector, a part (a page of inputs) and a tile cost something on
-        // top of the bytes.
-        std::vector<int64_t> cost(count);
+        // of about the same cost, so that a team of hmvm_dmma_kernel adds up the
+        // parts of a tile that it gets.  A vector, a part (a page of inputs) and a
+        // tile cost something on top of the bytes.
+        std::vector<int64_t> cost(count), run_cost(count);
         for (int32_t k = 0; k < count; k++) {
           const Item &it = items[first + k];
-          cost[k] = (int64_t)(it.vb - it.va) * 16 * (tb[it.tile].nrows + kItemVecRows) + kDmmaPartCost +
-                    (it.va == 0 ? kDmmaTileCost : 0);
+          cost[k] = it.cost;
+          run_cost[k] = (int64_t)(it.vb - it.va) * 16 * (tb[it.tile].nrows + kItemVecRows) + kDmmaPartCost +
+                        (it.va == 0 ? kDmmaTileCost : 0);
         }
         order = idx;
         team_begin = even_ranges(cost, nteams);
+        run_begin = even_ranges(run_cost, L.num_sms * kDmmaWarpsPerSm);
         return;
       }
       // largest first; by bytes alone where no team gets a second item
@@ -666,9 +672,10 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
       order.resize(count);
       for (int32_t k = 0; k < count; k++) order[pos[team_of[k]]++] = first + k;  // item order within team
     };
-    std::vector<int32_t> ord1, ord2, tb1, tb2;
-    assign(0, ni1, L.stage1_teams, ord1, tb1);
-    assign(ni1, ni2, L.stage2_teams, ord2, tb2);
+    std::vector<int32_t> ord1, ord2, tb1, tb2, rb1, rb2;
+    assign(0, ni1, L.stage1_teams, ord1, tb1, rb1);
+    assign(ni1, ni2, L.stage2_teams, ord2, tb2, rb2);
+    for (int32_t &b : rb2) b += ni1;
     std::vector<int32_t> order;
     order.reserve(items.size());
     order.insert(order.end(), ord1.begin(), ord1.end());
@@ -720,7 +727,7 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
       // one tile within one team.  A tile of one run needs no partial sums; the
       // others' runs write theirs at their first part's place.
       for (int st = 0; st < 2; st++) {
-        const std::vector<int32_t> &tbeg = st == 0 ? L.team_begin1 : L.team_begin2;
+        const std::vector<int32_t> &tbeg = st == 0 ? rb1 : rb2;  // items of each team of the kernel
         std::vector<int32_t> &mbeg = st == 0 ? L.mteam_begin1 : L.mteam_begin2;
         std::vector<int32_t> &red = st == 0 ? L.mred1 : L.mred2;
         int32_t tile = -1, nruns = 0;  // the tile of the last run and its runs so far

@@ -25,8 +25,10 @@
 //    vector ranges (segments trimmed to the range) that write partial sums; a
 //    small reduction adds the parts in order into t (stage 1) or y (stage 2).
 //  * Items are assigned to persistent "teams" (a warp, or a group of warps) by
-//    LPT on their byte cost and stored in team order, so a team streams one
-//    contiguous region of HBM.
+//    LPT on their cost and stored in team order, so a team streams one
+//    contiguous region of HBM.  FP64 and FP32 plans for several right-hand sides
+//    store them in tile order instead, and each kernel's teams get consecutive
+//    ranges of about the same cost.
 #pragma once
 
 #include <cstdint>

@@ -478,12 +478,14 @@ int hmvm_b200_layout_build_d(const hmvm_matrix2_d *mat2, const hmvm_plan_opts *o
                              hmvm_layout **layout);
 int hmvm_b200_layout_build64(const hmvm_leaves64 *lv, int32_t rowmat_is_float, const hmvm_plan_opts *opts,
                              int32_t num_sms, hmvm_layout **layout);
-/* Bounds checks of every descriptor of a single-vector layout against the
- * buffers it indexes: each item's data-stream range, segment range, rows, the
- * x or t columns of its segments, its padded inputs against the stage kernel's
- * input buffer, the y / t / partial-sum rows it writes, its t slots and row
- * scales, every reduction entry, and the team ranges.  HMVM_OK, or HMVM_ERANGE
- * with a message naming the first failing item.  Wide tensor-core layouts
+/* Bounds checks of every descriptor of a layout against the buffers it indexes:
+ * each item's data-stream range, segment range, rows, the x or t columns of its
+ * segments, its padded inputs against the stage kernel's input buffer, the y / t /
+ * partial-sum rows it writes, its t slots and row scales, every reduction entry,
+ * and the team ranges; that the items cover the data stream in order, and that
+ * every y row and partial sum is written once and every partial sum read once.
+ * The multi-RHS items of hmvm_b200_layout_multi_view likewise.  HMVM_OK, or
+ * HMVM_ERANGE with a message naming the first failing item.  Wide tensor-core layouts
  * (view.tcw = 1) are not described by these checks and return HMVM_OK.  The
  * library built with HMVM_DEVICE_CHECKS (libhmvm_b200_checked.so) runs the same
  * checks at plan creation and on the device before every single-vector stage
@@ -493,12 +495,28 @@ int hmvm_b200_layout_build64(const hmvm_leaves64 *lv, int32_t rowmat_is_float, c
  * arrays directly). */
 int hmvm_b200_layout_validate(const hmvm_layout *layout);
 /* The device address of a plan's item descriptors (hmvm_tile_desc[n_tiles],
- * stage-1 items first), for inspection and for tests of the device checks;
+ * stage-1 items first; those of its single-vector kernels), for inspection and for tests of the device checks;
  * a caller that changes them owns the consequences (the HMVM_DEVICE_CHECKS
  * build reports descriptors that leave their buffers instead of following
  * them). */
 int hmvm_b200_plan_descriptors(const hmvm_plan *plan, void **tiles_dev, int32_t *n_tiles, int32_t *stage1_tiles);
 int hmvm_b200_layout_view(const hmvm_layout *layout, hmvm_layout_view *view);
+/* The items that the multi-RHS kernel of FP64 and FP32 plans (nrhs_max 2..8)
+ * runs over the same data stream, t slots and partial sums: each the consecutive
+ * parts of one tile that a team has.  All zero for other layouts. */
+typedef struct hmvm_layout_multi_view {
+  int32_t n_tiles, n_segs;
+  int32_t stage1_tiles;                /* tiles [0,stage1) are stage 1, then stage 2 */
+  int32_t stage1_teams, stage2_teams;
+  int32_t n_red1, n_red2, _pad0;
+  const void *tiles;                   /* hmvm_tile_desc[n_tiles] */
+  const void *segs;                    /* hmvm_seg_desc[n_segs] */
+  const int32_t *seg_first;            /* [n_segs]: a segment's first padded column within its item */
+  const int32_t *team_begin1;          /* [stage1_teams+1], indexes tiles */
+  const int32_t *team_begin2;          /* [stage2_teams+1], indexes tiles */
+  const int32_t *red1, *red2;          /* as in hmvm_layout_view, 4 values per entry */
+} hmvm_layout_multi_view;
+int hmvm_b200_layout_multi_view(const hmvm_layout *layout, hmvm_layout_multi_view *view);
 void hmvm_b200_layout_destroy(hmvm_layout *layout);
 
 /* ---- misc --------------------------------------------------------------- */
