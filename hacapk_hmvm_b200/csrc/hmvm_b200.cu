@@ -2283,7 +2283,7 @@ int batch_create(const std::vector<LeafTable>& tabs, bool is_float, const hmvm_p
   std::sort(order.begin(), order.end());
   order.erase(std::unique(order.begin(), order.end()), order.end());
   std::vector<double> elems;
-  double wsum = 0;
+  std::vector<int> npass;
   for (int key : order) {
     BatchClass c;
     c.width = multi_inst_width(o.precision, key / 1024);
@@ -2296,30 +2296,11 @@ int batch_create(const std::vector<LeafTable>& tabs, bool is_float, const hmvm_p
       c.members.push_back(m);
       el += (double)std::max<int64_t>(tabs[m].len, 1);
     }
-    wsum += el * c.npass;
+    npass.push_back(c.npass);
     b->cls.push_back(std::move(c));
     elems.push_back(el);
   }
-  // Whole SMs per class, all passes together no more than there are: rounding to
-  // the nearest could ask for one SM too many, and the CTAs of a second wave made
-  // the launch 1.7 times as long.  The SMs left over go where most is missing.
-  std::vector<int> share(b->cls.size());
-  int left = sms;
-  auto want = [&](size_t k) { return sms * elems[k] / std::max(wsum, 1.0); };
-  for (size_t k = 0; k < share.size(); k++) {
-    share[k] = std::max(1, std::min(sms, (int)want(k)));
-    left -= share[k] * b->cls[k].npass;
-  }
-  for (;;) {
-    int best = -1;
-    for (size_t k = 0; k < share.size(); k++)
-      if (b->cls[k].npass <= left && want(k) > share[k] &&
-          (best < 0 || want(k) - share[k] > want(best) - share[best]))
-        best = (int)k;
-    if (best < 0) break;
-    share[best]++;
-    left -= b->cls[best].npass;
-  }
+  const std::vector<int> share = sm_shares(elems, npass, sms);
   for (size_t k = 0; k < b->cls.size(); k++) {
     int rc = class_create(b->cls[k], tabs, is_float, o, share[k]);
     if (rc) {

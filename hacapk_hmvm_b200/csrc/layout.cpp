@@ -160,6 +160,39 @@ std::vector<int32_t> even_ranges(const std::vector<int64_t> &cost, int n) {
   return out;
 }
 
+std::vector<int> sm_shares(const std::vector<double> &work, const std::vector<int> &npass, int sms) {
+  const size_t n = work.size();
+  double total = 0;
+  for (size_t k = 0; k < n; k++) total += work[k] * npass[k];
+  auto want = [&](size_t k) { return sms * work[k] / std::max(total, 1.0); };
+  std::vector<int> share(n);
+  int left = sms;
+  for (size_t k = 0; k < n; k++) {
+    share[k] = std::max(1, std::min(sms, (int)want(k)));
+    left -= share[k] * npass[k];
+  }
+  // small classes got a whole SM: take theirs from the class that misses one least
+  while (left < 0) {
+    int best = -1;
+    for (size_t k = 0; k < n; k++)
+      if (share[k] > 1 && (best < 0 || (share[k] - 1) * want(best) > (share[best] - 1) * want(k))) best = (int)k;
+    if (best < 0) break;  // more passes than SMs
+    share[best]--;
+    left += npass[best];
+  }
+  // the SMs left over go where most is missing
+  for (;;) {
+    int best = -1;
+    for (size_t k = 0; k < n; k++)
+      if (npass[k] <= left && want(k) > share[k] && (best < 0 || want(k) - share[k] > want(best) - share[best]))
+        best = (int)k;
+    if (best < 0) break;
+    share[best]++;
+    left -= npass[best];
+  }
+  return share;
+}
+
 int default_stage_cfg(int precision, int kernel, int stage) {
   if (precision == HMVM_MIXED) return stage == 1 ? kDefaultMixedCfg1 : kDefaultMixedCfg2;
   if (kernel == 0) return stage == 1 ? kDefaultStage1Cfg : kDefaultStage2Cfg;

@@ -313,6 +313,12 @@ int validate_leaves(const LeafTable &lt, std::string &msg);
 // ranges may be empty).
 std::vector<int32_t> even_ranges(const std::vector<int64_t> &cost, int n);
 
+// Whole SMs for each class of a batch, in proportion to its work (of one pass; it
+// runs npass of them side by side, each on its own SMs): at least one, and all
+// passes together no more than sms unless there are more passes than SMs.  The CTAs
+// that did not fit ran as a second wave, which made a launch 1.7 times as long.
+std::vector<int> sm_shares(const std::vector<double> &work, const std::vector<int> &npass, int sms);
+
 // The wide tensor-core layout (see layout_tc.cpp).
 int build_tc_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, HostLayout &out,
                     std::string &msg);
