@@ -147,6 +147,19 @@ __global__ void axpbyz(T* __restrict__ z, const T* __restrict__ x, double a, con
   }
 }
 
+// Launches a kernel and reports a failed launch at once: the workspace outlives a
+// solve, so a scalar that a kernel did not write would be an earlier solve's.
+template <typename... P, typename... A>
+int launch(cudaStream_t st, void (*kernel)(P...), dim3 grid, int threads, A... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3((unsigned)threads);
+  c.stream = st;
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+  return e == cudaSuccess ? HMVM_OK : set_error(HMVM_ECUDA, std::string("solver kernel: ") + cudaGetErrorString(e));
+}
+int copied(cudaError_t e) { return e == cudaSuccess ? HMVM_OK : set_error(HMVM_ECUDA, "solver: vector copy"); }
+
 template <typename T>
 struct Solver {
   hmvm_plan* plan;
@@ -156,8 +169,9 @@ struct Solver {
   double host[2];
 
   int dot2(const T* x0, const T* y0, const T* x1, const T* y1, double* d0, double* d1) {
-    dot2_partial<T><<<kDotBlocks, kDotThreads, 0, st>>>(x0, y0, x1, y1, n, part);
-    dot2_final<<<1, kDotBlocks, 0, st>>>(part, kDotBlocks, part + 2 * kDotBlocks);
+    int rc = launch(st, dot2_partial<T>, kDotBlocks, kDotThreads, x0, y0, x1, y1, n, part);
+    if (!rc) rc = launch(st, dot2_final, 1, kDotBlocks, part, kDotBlocks, part + 2 * kDotBlocks);
+    if (rc) return rc;
     if (cudaMemcpyAsync(host, part + 2 * kDotBlocks, 2 * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
       return set_error(HMVM_ECUDA, "bicgstab: inner products");
@@ -165,8 +179,8 @@ struct Solver {
     if (d1) *d1 = host[1];
     return HMVM_OK;
   }
-  void lin(T* z, const T* x, double a, const T* y, double b = 0.0, const T* w = nullptr) {
-    axpbyz<T><<<(n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184, 256, 0, st>>>(z, x, a, y, b, w, n);
+  int lin(T* z, const T* x, double a, const T* y, double b = 0.0, const T* w = nullptr) {
+    return launch(st, axpbyz<T>, (n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184, 256, z, x, a, y, b, w, n);
   }
 };
 
@@ -319,11 +333,12 @@ int bicgstab_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, double e
   double bnorm = 0, relres = 0;
   int steps = 0;
   rc = hmvm_b200_apply(plan, u, akt, st);
-  if (!rc) bicg_start<T><<<kDotBlocks, kDotThreads, 0, st>>>(b, akt, r, sh, n, part0);
+  if (!rc) rc = launch(st, bicg_start<T>, kDotBlocks, kDotThreads, b, akt, r, sh, n, part0);
   for (int k = 0; !rc; k++) {
     // the next direction; its record tells how the step before it ended
     BicgState *in = state + (k & 1 ? 0 : 1), *out = state + (k & 1 ? 1 : 0);
-    bicg_direction<T><<<kDotBlocks, kDotThreads, 0, st>>>(r, akp, p, n, k == 0, part0, in, out);
+    rc = launch(st, bicg_direction<T>, kDotBlocks, kDotThreads, r, akp, p, n, k == 0, part0, in, out);
+    if (rc) break;
     if (cudaMemcpyAsync(&h, out, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess) {
       rc = set_error(HMVM_ECUDA, "bicgstab: inner products");
@@ -346,13 +361,11 @@ int bicgstab_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, double e
     }
     if (!(relres >= eps) || k >= max_steps) break;
     rc = hmvm_b200_apply(plan, p, akp, st);
-    if (rc) break;
-    dot2_partial<T><<<kDotBlocks, kDotThreads, 0, st>>>(sh, r, sh, akp, n, part1);
-    bicg_half<T><<<kDotBlocks, kDotThreads, 0, st>>>(r, akp, t, n, part1, out);
-    rc = hmvm_b200_apply(plan, t, akt, st);
-    if (rc) break;
-    dot2_partial<T><<<kDotBlocks, kDotThreads, 0, st>>>(akt, t, akt, akt, n, part2);
-    bicg_step<T><<<kDotBlocks, kDotThreads, 0, st>>>(u, r, p, t, akt, sh, n, part2, out, part0);
+    if (!rc) rc = launch(st, dot2_partial<T>, kDotBlocks, kDotThreads, sh, r, sh, akp, n, part1);
+    if (!rc) rc = launch(st, bicg_half<T>, kDotBlocks, kDotThreads, r, akp, t, n, part1, out);
+    if (!rc) rc = hmvm_b200_apply(plan, t, akt, st);
+    if (!rc) rc = launch(st, dot2_partial<T>, kDotBlocks, kDotThreads, akt, t, akt, akt, n, part2);
+    if (!rc) rc = launch(st, bicg_step<T>, kDotBlocks, kDotThreads, u, r, p, t, akt, sh, n, part2, out, part0);
   }
   cudaStreamSynchronize(st);
   if (!kept) cudaFree(ws);
@@ -381,11 +394,9 @@ int gcrm_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, int m, doubl
   int steps = 0;
   // r = b - A u; p_0 = r
   rc = hmvm_b200_apply(plan, u, ar, st);
-  if (!rc) {
-    s.lin(r, b, -1.0, ar);
-    cudaMemcpyAsync(p, r, sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
-    rc = s.dot2(b, b, r, r, &bb, &rr);
-  }
+  if (!rc) rc = s.lin(r, b, -1.0, ar);
+  if (!rc) rc = copied(cudaMemcpyAsync(p, r, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));
+  if (!rc) rc = s.dot2(b, b, r, r, &bb, &rr);
   const double bnorm = std::sqrt(bb);
   relres = bnorm > 0 ? std::sqrt(rr) / bnorm : 0.0;
   if (!rc && relres >= eps && max_steps > 0) rc = hmvm_b200_apply(plan, p, ap, st);  // ap_0 = A p_0
@@ -401,22 +412,22 @@ int gcrm_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, int m, doubl
     }
     capap[ik] = qq;
     const double alpha = nom / qq;
-    s.lin(u, u, alpha, p + (size_t)ik * ld);  // u += alpha p_ik
-    s.lin(r, r, -alpha, q);                   // r -= alpha ap_ik
-    rc = s.dot2(r, r, nullptr, nullptr, &rr, nullptr);
+    rc = s.lin(u, u, alpha, p + (size_t)ik * ld);  // u += alpha p_ik
+    if (!rc) rc = s.lin(r, r, -alpha, q);          // r -= alpha ap_ik
+    if (!rc) rc = s.dot2(r, r, nullptr, nullptr, &rr, nullptr);
     if (rc) break;
     relres = std::sqrt(rr) / bnorm;
     steps = in;
     if (relres < eps || in == max_steps) break;
     rc = hmvm_b200_apply(plan, r, ar, st);  // ar = A r
-    if (rc) break;
     const int ikn = in % m;
-    cudaMemcpyAsync(p + (size_t)ikn * ld, r, sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
-    cudaMemcpyAsync(ap + (size_t)ikn * ld, ar, sizeof(T) * n, cudaMemcpyDeviceToDevice, st);
+    if (!rc) rc = copied(cudaMemcpyAsync(p + (size_t)ikn * ld, r, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));
+    if (!rc) rc = copied(cudaMemcpyAsync(ap + (size_t)ikn * ld, ar, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));
     // beta_il = -(ap_il . ar) / capap_il for il = 0..ik, all against the same ar
     const int k = ik + 1;
-    dotm_partial<T><<<dim3(kDotBlocks, k), kDotThreads, 0, st>>>(ap, ld, ar, n, part);
-    dotm_final<<<k, kDotBlocks, 0, st>>>(part, kDotBlocks, dots);
+    if (!rc) rc = launch(st, dotm_partial<T>, dim3(kDotBlocks, k), kDotThreads, ap, ld, ar, n, part);
+    if (!rc) rc = launch(st, dotm_final, k, kDotBlocks, part, kDotBlocks, dots);
+    if (rc) break;
     if (cudaMemcpyAsync(hd.data(), dots, sizeof(double) * k, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess) {
       rc = set_error(HMVM_ECUDA, "gcrm: inner products");
@@ -424,7 +435,7 @@ int gcrm_t(hmvm_plan* plan, int n, const T* b, T* u, int max_steps, int m, doubl
     }
     Betas be;
     for (int il = 0; il < k; il++) be.b[il] = -hd[il] / capap[il];
-    gcr_update<T><<<(n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184, 256, 0, st>>>(p, ap, ld, k, ikn, be, n);
+    rc = launch(st, gcr_update<T>, (n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184, 256, p, ap, ld, k, ikn, be, n);
   }
   cudaStreamSynchronize(st);
   if (!kept) cudaFree(ws);
