@@ -672,7 +672,7 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
         std::vector<int64_t> cost(count), run_cost(count);
         for (int32_t k = 0; k < count; k++) {
           const Item &it = items[first + k];
-          cost[k] = it.cost;
+          cost[k] = (int64_t)(it.vb - it.va) * 16 * (tb[it.tile].nrows + kRangeVecRows) + kRangeItemBytes;
           run_cost[k] = (int64_t)(it.vb - it.va) * 16 * (tb[it.tile].nrows + kItemVecRows) + kDmmaPartCost +
                         (it.va == 0 ? kDmmaTileCost : 0);
         }

@@ -129,6 +129,16 @@ constexpr int64_t kItemsPerTeam = 6;
 // 54.8 us; by bytes and 1 KiB alone 59.5.  N = 131,072 mixed: 196.5 against 203.1 us.
 constexpr int kItemVecRows = 8, kItemVecRowsMixed = 16;
 constexpr int64_t kItemOverheadBytes = 4096;
+// The same for the single-vector kernels' ranges of consecutive items (plain plans
+// for several right-hand sides).  Neighbouring items are alike, so what the cost
+// gets wrong adds up within a team.  Whole apply, N = 90,001 FP64, nrhs_max 8 (and
+// 2), with 8 rows and 4 KiB: 349 (302) us; 16 rows and 4 KiB 319 (291); 8 rows and
+// 16 KiB 311 (291); 16 rows and 16 KiB 303 (285); 16 rows and 32 KiB 304 (285); LPT
+// over items stored in team order 299 (281).  A share per segment, or ranges of
+// tiles taken from all over the matrix, changed nothing.  nrhs_max 8, FP32: 184 ->
+// 177 (LPT 190); FP64 N = 30,001: 97.5 -> 88.7 (90.0), N = 10,000: 46.0 -> 41.2 (41.1).
+constexpr int kRangeVecRows = 16;
+constexpr int64_t kRangeItemBytes = 16384;
 
 // Element type of a segment's matrix data (mixed-precision plans encode it in
 // the top bits of hmvm_seg_desc.ncols; plain plans leave those bits zero).
