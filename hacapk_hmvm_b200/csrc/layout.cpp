@@ -673,7 +673,7 @@ int build_layout(const LeafTable &lt, const hmvm_plan_opts &opts, int num_sms, H
         for (int32_t k = 0; k < count; k++) {
           const Item &it = items[first + k];
           cost[k] = (int64_t)(it.vb - it.va) * 16 * (tb[it.tile].nrows + kRangeVecRows) + kRangeItemBytes;
-          run_cost[k] = (int64_t)(it.vb - it.va) * 16 * (tb[it.tile].nrows + kItemVecRows) + kDmmaPartCost +
+          run_cost[k] = (int64_t)(it.vb - it.va) * 16 * (tb[it.tile].nrows + kItemVecRows) + dmma_part_cost(nrhs_max) +
                         (it.va == 0 ? kDmmaTileCost : 0);
         }
         order = idx;

@@ -216,10 +216,16 @@ constexpr int kDmmaPageBytes = 4096;
 constexpr int kDmmaRingPad = 512;
 constexpr int kDmmaWarpsPerSm = 12;
 // Cost of an item's part in bytes when its teams get their ranges: its vectors of
-// nrows + kItemVecRows rows, kDmmaPartCost, and kDmmaTileCost for a tile's first
+// nrows + kItemVecRows rows, dmma_part_cost, and kDmmaTileCost for a tile's first
 // part.  V stage of 8 FP32 right-hand sides (N = 100,003): 86 us; with 4 KiB less
-// per tile 105, with 8 KiB more 95, without the rows' share 112.
-constexpr int64_t kDmmaPartCost = 2048, kDmmaTileCost = 4096;
+// per tile 105, without the rows' share 112, with 4 KiB more per tile 90.  Parts of
+// plans up to 4 wide hold up to twice the vectors (they are cut by their inputs'
+// bytes) and fill more pages.  Whole applies with 2 and 4 KiB per part, up to 4 wide:
+// FP32 N = 30,001 x 4 83.2 and 81.4 us, N = 15,000 x 2 51.7 and 50.1, N = 10,000 x 2
+// 46.6 and 45.7; FP64 N = 30,001 x 4 105.0 and 104.5, x 2 103.6 and 102.9.  8 wide: FP32
+// N = 100,003 251.5 and 251.6, N = 30,001 81.5 and 82.5; FP64 N = 65,536 214.7 and 215.6.
+constexpr int64_t kDmmaTileCost = 4096;
+constexpr int64_t dmma_part_cost(int nrhs_max) { return nrhs_max <= 4 ? 4096 : 2048; }
 constexpr int dmma_smem_bytes(const MultiCfg& c) {
   return c.wpb * (c.slots * c.chunk + kDmmaRingPad + 2 * kDmmaPageBytes + (c.slots + 2) * 8);
 }
