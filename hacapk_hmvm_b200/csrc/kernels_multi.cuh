@@ -1,16 +1,15 @@
-// Multi-RHS HMVM on the CUDA cores: Y = H X for NR right-hand sides per pass
-// (NR in {1, 2, 4, 8}), over the same planner layout as the single-vector
-// kernels (hmvm_reduce_kernel / hmvm_stream_kernel / hmvm_mixed_kernel).
+// Multi-RHS HMVM: Y = H X for NR right-hand sides per pass (2, 4 or 8, and the 16
+// of kernels_tc.cuh), over the planner's layout of the single-vector kernels.
 //
 //   hmvm_pack_x_kernel      X (column-major, leading dimension ldx) -> the
 //                           row-interleaved input xpk[i * NR + r] (FP64 and/or
 //                           FP32 copies, zero rows past N), so that every
 //                           segment's inputs are one contiguous block.
-//   hmvm_multi_kernel       mixed plans (plain plans: kernels_dmma.cuh): one
-//                           warp per team, lane = row; the matrix streams
-//                           through the warp's TMA ring exactly as in the
-//                           single-vector kernels; each stored element is
-//                           multiplied by its column's NR inputs.  V stage:
+//   hmvm_multi_kernel       mixed plans, on the CUDA cores (plain plans:
+//                           kernels_dmma.cuh): one warp per team, lane = row;
+//                           the matrix streams through the warp's TMA ring as
+//                           in the single-vector kernels; each stored element
+//                           is multiplied by its column's NR inputs.  V stage:
 //                           t[slot * NR + r]; row stage: Y[row + r * ldy] or
 //                           partial sums p[(base + lane) * NR + r].
 //   hmvm_reduce_multi_kernel adds the partial sums of split tiles in part
@@ -108,8 +107,8 @@ struct MultiMode {
 };
 
 // Copy the inputs item `d` reads into zb: for each segment, ncp columns of
-// NR values (ncp = columns rounded up to whole vectors; the padding is zero).
-// FP64 segments take 8-byte values, the others 4-byte values.
+// NR (even) values (ncp = columns rounded up to whole vectors; the padding is
+// zero).  FP64 segments take 8-byte values, the others 4-byte values.
 template <int NR, bool CHECK = false>
 __device__ __forceinline__ void gather_multi(const hmvm_tile_desc& d, const hmvm_seg_desc& sreg, const MultiArgs& a,
                                              unsigned char* zb, int lane) {
@@ -133,16 +132,9 @@ __device__ __forceinline__ void gather_multi(const hmvm_tile_desc& d, const hmvm
     if (type == kF64) {
       const double* s = a.x64 + base;  // FP64 segments are dense leaves
       double* z = reinterpret_cast<double*>(zb + zoff);
-      if constexpr (NR % 2 == 0) {  // 16-byte copies: (src * NR) is even
-        for (int c = lane; c < ncp * NR / 2; c += 32) {
-          if (c < nc * NR / 2) cp_async<16>(z + 2 * c, s + 2 * c);
-          else *reinterpret_cast<double2*>(z + 2 * c) = make_double2(0.0, 0.0);
-        }
-      } else {
-        for (int c = lane; c < ncp; c += 32) {
-          if (c < nc) cp_async<8>(z + c, s + c);
-          else z[c] = 0.0;
-        }
+      for (int c = lane; c < ncp * NR / 2; c += 32) {  // 16-byte copies: (src * NR) is even
+        if (c < nc * NR / 2) cp_async<16>(z + 2 * c, s + 2 * c);
+        else *reinterpret_cast<double2*>(z + 2 * c) = make_double2(0.0, 0.0);
       }
       zoff += ncp * NR * 8;
     } else {
@@ -153,15 +145,11 @@ __device__ __forceinline__ void gather_multi(const hmvm_tile_desc& d, const hmvm
           if (c < nc * NR / 4) cp_async<16>(z + 4 * c, s + 4 * c);
           else *reinterpret_cast<float4*>(z + 4 * c) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-      } else if constexpr (NR == 2) {
+      } else {
+        static_assert(NR == 2, "passes of 2, 4, 8 or 16 right-hand sides");
         for (int c = lane; c < ncp; c += 32) {
           if (c < nc) cp_async<8>(z + 2 * c, s + 2 * c);
           else *reinterpret_cast<float2*>(z + 2 * c) = make_float2(0.f, 0.f);
-        }
-      } else {
-        for (int c = lane; c < ncp; c += 32) {
-          if (c < nc) cp_async<4>(z + c, s + c);
-          else z[c] = 0.f;
         }
       }
       zoff += ncp * NR * 4;
@@ -181,24 +169,18 @@ __device__ __forceinline__ void axpy_f(float* acc, float a, const float* z) {
       fma2(acc[4 * q + 0], acc[4 * q + 1], aa, make_float2(zz.x, zz.y));
       fma2(acc[4 * q + 2], acc[4 * q + 3], aa, make_float2(zz.z, zz.w));
     }
-  } else if constexpr (NR == 2) {
+  } else {
     const float2 zz = *reinterpret_cast<const float2*>(z);
     fma2(acc[0], acc[1], aa, zz);
-  } else {
-    acc[0] = fmaf(a, z[0], acc[0]);
   }
 }
 template <int NR>
 __device__ __forceinline__ void axpy_d(double* acc, double a, const double* z) {
-  if constexpr (NR >= 2) {
 #pragma unroll
-    for (int q = 0; q < NR / 2; q++) {
-      const double2 zz = reinterpret_cast<const double2*>(z)[q];
-      acc[2 * q + 0] = fma(a, zz.x, acc[2 * q + 0]);
-      acc[2 * q + 1] = fma(a, zz.y, acc[2 * q + 1]);
-    }
-  } else {
-    acc[0] = fma(a, z[0], acc[0]);
+  for (int q = 0; q < NR / 2; q++) {
+    const double2 zz = reinterpret_cast<const double2*>(z)[q];
+    acc[2 * q + 0] = fma(a, zz.x, acc[2 * q + 0]);
+    acc[2 * q + 1] = fma(a, zz.y, acc[2 * q + 1]);
   }
 }
 

@@ -181,8 +181,8 @@ int default_stage_cfg(int precision, int kernel, int stage);
 constexpr int kDefaultMixedCfg1 = 10;
 constexpr int kDefaultMixedCfg2 = 8;
 
-// Multi-RHS kernel (hmvm_multi_kernel): rhs per pass and its input buffer.
-constexpr int kMaxNrhsPass = 8;   // CUDA-core multi-RHS passes
+// Multi-RHS kernels: right-hand sides per pass and input buffers.
+constexpr int kMaxNrhsPass = 8;    // widest pass of hmvm_dmma_kernel and hmvm_multi_kernel
 constexpr int kTcNrhs = 16;        // tensor-core passes (mixed plans with nrhs_max = 16)
 constexpr int kTcWarpsPerSm = 7;   // resident warps (teams) per SM of the tensor-core kernel
 // Each warp's two input buffers of hmvm_multi_kernel (an item's x/t columns for
