@@ -12,10 +12,10 @@
 // adds up the partial sums itself, and the host reads one record per step, for
 // the stopping test ||r|| / ||b|| < eps.  GCR(m) reads its inner products back.
 //
-// BiCGSTAB at N = 12,000 (FP64, 7 steps, 15 products of 45 us): 2.1 to 5.5 ms
-// (the allocator's share varies) with work vectors allocated and freed by each
-// call and three round trips to the host per step, 0.86 ms with the plan's
-// workspace and one.  What is left is the products and the gaps before them.
+// BiCGSTAB at N = 12,000 (FP64, 7 steps, 15 products of 45 us): 2.1 ms with work
+// vectors allocated and freed by each call (more where the allocator is slow) and
+// three round trips to the host per step, 0.70 to 0.86 ms with the plan's workspace
+// and one.  What is left is the products and the gaps before them.
 #include <cuda_runtime.h>
 
 #include <cmath>
